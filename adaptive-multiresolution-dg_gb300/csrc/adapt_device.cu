@@ -30,6 +30,7 @@
 
 #include "amdg_internal.hpp"
 #include "kernels.cuh"
+#include "kernels_plan.cuh"
 #include "device_alloc.cuh"
 
 using namespace amdg;
@@ -624,12 +625,14 @@ __device__ __forceinline__ void row_lists(const TopoArgs& A, int64_t e, int t, c
     *sf_out = sf;
 }
 
-__global__ void topo_count_kernel(TopoArgs A, int32_t* __restrict__ vcnt, int32_t* __restrict__ fcnt) {
+__global__ void topo_count_kernel(TopoArgs A, int32_t* __restrict__ vcnt, int32_t* __restrict__ fcnt,
+                                  int32_t* __restrict__ long_count) {
     const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int dim = A.ks.dim;
     if (row > A.E * dim) return;  // whole warps: the row test is uniform
     if (row == A.E * dim) {
         if ((threadIdx.x & 31) == 0) vcnt[row] = fcnt[row] = 0;
+        if ((threadIdx.x & 31) < kMaxDim) long_count[threadIdx.x & 31] = 0;  // the fill kernel appends
         return;
     }
     const int64_t e = row / dim;
@@ -643,14 +646,20 @@ __global__ void topo_count_kernel(TopoArgs A, int32_t* __restrict__ vcnt, int32_
 
 __global__ void topo_fill_kernel(TopoArgs A, const int32_t* __restrict__ vol_ptr, const int32_t* __restrict__ flx_ptr,
                                  int2* __restrict__ vol_nbr, int2* __restrict__ flx_nbr, int32_t* __restrict__ vol_split,
-                                 int32_t* __restrict__ flx_split, int64_t vol_cap, int64_t flx_cap, int* err) {
+                                 int32_t* __restrict__ flx_split, int64_t vol_cap, int64_t flx_cap, int* err,
+                                 RowRec* __restrict__ rows, int32_t* long_count, int32_t* long_rows,
+                                 int64_t long_stride) {
     const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int dim = A.ks.dim;
     if (row >= A.E * dim) return;
     const int64_t v0 = vol_ptr[row], f0 = flx_ptr[row];
     const int64_t v1 = vol_ptr[row + 1], f1 = flx_ptr[row + 1];
     if (v1 > vol_cap || f1 > flx_cap) {  // lists beyond the arrays: write nothing
-        if ((threadIdx.x & 31) == 0) atomicOr(err, 1);
+        if ((threadIdx.x & 31) == 0) {
+            atomicOr(err, 1);
+            const int o = A.ks.field(A.keys[row / dim], int(row % dim));
+            write_row_rec(rows, row, dim, 0, 0, 0, 0, 0, 0, o, long_count, long_rows, long_stride);
+        }
         return;
     }
     const RowOut out{vol_nbr + v0, flx_nbr + f0, v1 - v0, f1 - f0};
@@ -661,6 +670,8 @@ __global__ void topo_fill_kernel(TopoArgs A, const int32_t* __restrict__ vol_ptr
         if (nv != v1 - v0 || nf != f1 - f0) atomicOr(err, 1);
         vol_split[row] = int32_t(v0 + sv);
         flx_split[row] = int32_t(f0 + sf);
+        write_row_rec(rows, row, dim, int(v0), int(v0 + sv), int(v1), int(f0), int(f0 + sf), int(f1),
+                      A.ks.field(A.keys[e], int(row - e * dim)), long_count, long_rows, long_stride);
     }
 }
 
@@ -1190,7 +1201,7 @@ amdg_status device_transform_topology(amdg_grid* g, const DeviceTopoOut& out, in
     // counts of the vol rows in d_cnt[0 .. rows], of the flx rows in d_cnt[rows + 1 ..]
     int32_t* vcnt = d_cnt;
     int32_t* fcnt = d_cnt + rows + 1;
-    topo_count_kernel<<<blocks_for(32 * (rows + 1), 256), 256, 0, st>>>(A, vcnt, fcnt);
+    topo_count_kernel<<<blocks_for(32 * (rows + 1), 256), 256, 0, st>>>(A, vcnt, fcnt, out.long_count);
     AMDG_CK(cudaGetLastError());
     if (rows + 1 <= kSmallCoarsenMax) {
         scan_pair_small_kernel<<<1, kSmallCoarsenThreads, 0, st>>>(vcnt, fcnt, rows + 1, out.vol_ptr, out.flx_ptr);
@@ -1206,7 +1217,8 @@ amdg_status device_transform_topology(amdg_grid* g, const DeviceTopoOut& out, in
     }
     topo_fill_kernel<<<blocks_for(32 * rows, 256), 256, 0, st>>>(
         A, out.vol_ptr, out.flx_ptr, reinterpret_cast<int2*>(out.vol_nbr), reinterpret_cast<int2*>(out.flx_nbr),
-        out.vol_split, out.flx_split, out.vol_cap, out.flx_cap, out.err);
+        out.vol_split, out.flx_split, out.vol_cap, out.flx_cap, out.err, static_cast<RowRec*>(out.rows), out.long_count,
+        out.long_rows, out.long_stride);
     AMDG_CK(cudaGetLastError());
     ancestors_kernel<<<blocks_for(rows, 128), 128, 0, st>>>(A, out.anc_order, out.p1, out.anc, out.err);
     AMDG_CK(cudaGetLastError());

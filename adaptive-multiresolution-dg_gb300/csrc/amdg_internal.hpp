@@ -247,6 +247,7 @@ constexpr int kMaxTermSources = kMaxDim + 1;  // inputs a term's first sweep can
 struct PartialSum {
     int8_t dims[kMaxDim], lu[kMaxDim], mat[kMaxDim], flx[kMaxDim];
     int8_t src;    // input of the first sweep (index into the launch's sources)
+    int8_t grp;    // terms that are only ever evaluated together (a term group, a point field)
     int32_t kind;
     double coef;
     // as a node of a launch's sweep tree: the slice of the previous sweep this node reads (sweeps
@@ -263,6 +264,30 @@ struct SweepTree {
 // nodes of the tree of terms [first, first + count) of `terms`, appended to `nodes`
 SweepTree build_sweep_tree(const std::vector<PartialSum>& terms, int first, int count, int dim,
                            std::vector<PartialSum>* nodes);
+// The sweeps of a range of terms as sums of products (kernels_plan.cu).  A product is one 1D
+// transform of an input: a source (first sweep), a node of the previous sweep, or (in < 0) the
+// Alpert coefficients (penalty).  A node is an element field, the sum of its products.  Within a
+// group, terms that end in the same transforms are added before these (the transforms are linear and
+// keep their order in every term); terms that begin alike share their nodes.  The last sweep has one
+// node, its products in the order of the groups, or one node per group (fields).
+struct PlanProduct {
+    int32_t in;
+    int8_t t, lu, flx, mat;
+    int32_t stride, in_block;  // of the input block: entries between indices along t, entries per element
+    double coef;
+};
+struct PlanNode {
+    int32_t first, count;  // products
+    int32_t long_dim;      // middle sweeps: the dimension of the products that are not "U" parts, -1 if none
+    int32_t long_mask;     // last sweep: the dimensions of those products, one bit each
+};
+struct SweepPlan {
+    int offset[kMaxDim] = {0}, count[kMaxDim] = {0};  // nodes of each sweep
+    int max_products = 0;                             // of a node of the last sweep
+};
+SweepPlan build_sweep_plan(const std::vector<PartialSum>& terms, int first, int count, int dim, int n_in, int n_out,
+                           int np, bool node_per_group, std::vector<PlanNode>* nodes,
+                           std::vector<PlanProduct>* products);
 // surplus ancestors: [e][d][ic] element index, ic < t.p1 (-1 for level 0 in d); false if a hole is found
 bool build_surplus_ancestors(const HostGrid& g, const LagrTables& t, std::vector<int32_t>* anc);
 
@@ -460,13 +485,24 @@ struct amdg_burgers_op {
     std::vector<amdg::PartialSum> nodes;
     amdg::PartialSum* d_nodes = nullptr;
     size_t nodes_cap = 0;
+    // sweep plans of the term ranges launched so far (the default sweeps), their nodes and products
+    std::vector<std::pair<std::pair<int, int>, amdg::SweepPlan>> plans;
+    std::vector<amdg::PlanNode> plan_nodes;
+    std::vector<amdg::PlanProduct> plan_products;
+    amdg::PlanNode* d_plan_nodes = nullptr;
+    amdg::PlanProduct* d_plan_products = nullptr;
+    size_t plan_nodes_cap = 0, plan_products_cap = 0;  // bytes
+    void* d_rows = nullptr;          // amdg::RowRec per (element, dimension)
+    int32_t* d_long = nullptr;       // long rows: counts per dimension (kMaxDim), then the elements per dimension
+    int64_t long_stride = 0;
+    double* d_sines = nullptr;       // wave: sin(2 pi x) of every 1D interpolation point
     int64_t interp_version = -1;     // element set of the flux coefficients amdg_lagr_interpolate kept
     int interp_prec = -1;            // ... and their arithmetic
     // wave: element set and arithmetic of the K grad u [0] and K u [1] interpolations amdg_wave_interpolate kept
     int64_t wave_interp_version[2] = {-1, -1};
     int wave_interp_prec[2] = {-1, -1};
     int chunk = 1;  // terms per launch
-    int sweep_variant = -1;  // transform sweep kernel: -1 by precision, 0 thread per output entry, 1 thread per
+    int sweep_variant = -1;  // transform sweep kernel: -1 the planned sweeps, else one sweep per term: 0 thread per output entry, 1 thread per
                              // column, 2 / 3 / 4 warp per (node, element) with 1 / 2 / 4 elements per warp
     // work buffers sized for FP64: E x p1^dim doubles each, the sweep buffers and
     // term slices chunk times that
@@ -558,6 +594,9 @@ struct DeviceTopoOut {
     const int32_t* anc_order;        // device [n1][p1]
     int p1;
     int* err;                        // device flag: a surplus ancestor is missing / a list overflowed
+    void* rows;                      // RowRec per (element, dimension) (kernels_plan.cuh)
+    int32_t *long_count, *long_rows; // long rows per dimension: counts, elements [dim][long_stride]
+    int64_t long_stride;
 };
 // bounds on the number of (element, neighbour) pairs of the vol and flx lists over all dimensions
 void transform_topology_bounds(const amdg_grid* g, int64_t* vol_pairs, int64_t* flx_pairs);

@@ -18,6 +18,7 @@
 #include "amdg_internal.hpp"
 #include "kernels.cuh"
 #include "kernels_lagr.cuh"
+#include "kernels_plan.cuh"
 #include "kernels_mlp.cuh"
 #include "device_alloc.cuh"
 
@@ -125,7 +126,7 @@ bool burgers_like(const amdg_burgers_op* op) { return op->kind == 0 || op->kind 
 
 // partial sums of the schedule with the given matrix and vol/flx choice per
 // dimension, reading input `src`, appended to op->terms
-void push_psums(amdg_burgers_op* op, const int* mat, const int* flx, double coef, int src) {
+void push_psums(amdg_burgers_op* op, const int* mat, const int* flx, double coef, int src, int grp) {
     const int dim = op->grid->host.dim;
     for (size_t s = 0; s < op->sched_dims.size(); ++s) {
         PartialSum p{};
@@ -137,6 +138,7 @@ void push_psums(amdg_burgers_op* op, const int* mat, const int* flx, double coef
             p.flx[j] = int8_t(flx[t]);
         }
         p.src = int8_t(src);
+        p.grp = int8_t(grp);
         p.kind = 0;
         p.coef = coef;
         op->terms.push_back(p);
@@ -147,6 +149,7 @@ void push_psums(amdg_burgers_op* op, const int* mat, const int* flx, double coef
 void push_penalty(amdg_burgers_op* op, int d, double coef) {
     PartialSum p{};
     p.dims[0] = int8_t(d);
+    p.grp = 3;
     p.kind = 1;
     p.coef = coef;
     op->terms.push_back(p);
@@ -180,12 +183,12 @@ void build_terms(amdg_burgers_op* op) {
     if (op->kind == 2) {  // interpolation init: u_v (Lagrange x Alpert) in every dimension
         op->n_pv_terms = 0;
         for (int t = 0; t < dim; ++t) { mat[t] = kMatLV; flx[t] = 0; }
-        push_psums(op, mat, flx, 1.0, 0);
+        push_psums(op, mat, flx, 1.0, 0, 0);
         return;
     }
     if (burgers_like(op)) {
         for (int t = 0; t < dim; ++t) { mat[t] = kMatA2P; flx[t] = 0; }
-        push_psums(op, mat, flx, 1.0, 0);
+        push_psums(op, mat, flx, 1.0, 0, 0);
         op->n_pv_terms = int(op->terms.size());
         // the three groups in the order the reference's driver calls them: rhs_vol_scalar (every
         // d), rhs_flx_intp_scalar (every d), rhs_flx_penalty_scalar (every d)
@@ -200,7 +203,7 @@ void build_terms(amdg_burgers_op* op) {
                     mat[t] = (t == d) ? (term == 0 ? kMatLVX : kMatLFLX) : kMatLV;
                     flx[t] = (term == 1 && t == d) ? 1 : 0;
                 }
-                push_psums(op, mat, flx, term == 0 ? 1.0 : 0.5, 0);
+                push_psums(op, mat, flx, term == 0 ? 1.0 : 0.5, 0, term);
             }
             op->grp_count[term] = int(op->terms.size()) - op->grp_first[term];
         }
@@ -208,20 +211,20 @@ void build_terms(amdg_burgers_op* op) {
     }
     for (int g = 0; g <= dim; ++g) {
         for (int t = 0; t < dim; ++t) { mat[t] = (t == g) ? kMatA2PD : kMatA2P; flx[t] = 0; }
-        push_psums(op, mat, flx, 1.0, 0);
+        push_psums(op, mat, flx, 1.0, 0, g);
     }
     op->n_pv_terms = int(op->terms.size());
     for (int d = 0; d < dim; ++d) {  // -{K u_x}[v]: uave_vjp = lflx / 2 exactly
         for (int t = 0; t < dim; ++t) { mat[t] = (t == d) ? kMatLFLX : kMatLV; flx[t] = (t == d) ? 1 : 0; }
-        push_psums(op, mat, flx, -0.5, d);
+        push_psums(op, mat, flx, -0.5, d, 0);
     }
     for (int d = 0; d < dim; ++d) {  // -K u_x v_x
         for (int t = 0; t < dim; ++t) { mat[t] = (t == d) ? kMatLVX : kMatLV; flx[t] = 0; }
-        push_psums(op, mat, flx, -1.0, d);
+        push_psums(op, mat, flx, -1.0, d, 1);
     }
     for (int d = 0; d < dim; ++d) {  // -1/2 [K u](v_x^- + v_x^+)
         for (int t = 0; t < dim; ++t) { mat[t] = (t == d) ? kMatLJV : kMatLV; flx[t] = (t == d) ? 1 : 0; }
-        push_psums(op, mat, flx, -0.5, dim);
+        push_psums(op, mat, flx, -0.5, dim, 2);
     }
     for (int d = 0; d < dim; ++d) push_penalty(op, d, 0.0);  // coefficient set per element set
 }
@@ -253,12 +256,49 @@ amdg_status upload_nodes(amdg_burgers_op* op, cudaStream_t st) {
     return AMDG_OK;
 }
 
-// after a change of term coefficients: the nodes of every tree again (the same structure: only
-// the penalty's coefficient changes, and the penalty is never shared)
+// the nodes and products of the sweep plans on the device
+amdg_status upload_plans(amdg_burgers_op* op, cudaStream_t st) {
+    auto up = [&](auto** dst, size_t* cap, const auto& host) -> amdg_status {
+        const size_t bytes = host.size() * sizeof(host[0]);
+        if (bytes > *cap) {
+            AMDG_CK(cudaStreamSynchronize(st));
+            cudaFree(*dst);
+            *dst = nullptr;
+            *cap = 0;
+            const size_t want = 2 * bytes + 4096;
+            if (amdg::device_malloc(reinterpret_cast<void**>(dst), want) != cudaSuccess)
+                return fail(AMDG_ERR_NOMEM, "cudaMalloc failed (sweep plans)");
+            *cap = want;
+            op->graph_version = -1;  // a captured step read the old buffer
+        }
+        if (bytes) AMDG_CK(cudaMemcpyAsync(*dst, host.data(), bytes, cudaMemcpyHostToDevice, st));
+        return AMDG_OK;
+    };
+    amdg_status s;
+    if ((s = up(&op->d_plan_nodes, &op->plan_nodes_cap, op->plan_nodes)) != AMDG_OK ||
+        (s = up(&op->d_plan_products, &op->plan_products_cap, op->plan_products)) != AMDG_OK)
+        return s;
+    AMDG_CK(cudaStreamSynchronize(st));  // the host vectors may change again before the copies would run
+    return AMDG_OK;
+}
+
+SweepPlan make_plan(amdg_burgers_op* op, int first, int count) {
+    const bool pv = first < op->n_pv_terms;
+    const int np = op->grid->host.k + 1;
+    return build_sweep_plan(op->terms, first, count, op->grid->host.dim, pv ? np : op->p1, pv ? op->p1 : np, np, pv,
+                            &op->plan_nodes, &op->plan_products);
+}
+
+// after a change of term coefficients: the nodes of every tree and plan again (the same structure:
+// only the penalty's coefficient changes, and the penalty is never shared)
 amdg_status refresh_nodes(amdg_burgers_op* op, cudaStream_t st) {
     op->nodes.clear();
     for (auto& kv : op->trees)
         kv.second = build_sweep_tree(op->terms, kv.first.first, kv.first.second, op->grid->host.dim, &op->nodes);
+    op->plan_nodes.clear();
+    op->plan_products.clear();
+    for (auto& kv : op->plans) kv.second = make_plan(op, kv.first.first, kv.first.second);
+    if (amdg_status s = upload_plans(op, st); s != AMDG_OK) return s;
     return upload_nodes(op, st);
 }
 
@@ -277,11 +317,55 @@ amdg_status sweep_tree(amdg_burgers_op* op, int first, int count, SweepTree* out
     return upload_nodes(op, st);
 }
 
+// the sweep plan of the same terms
+amdg_status sweep_plan(amdg_burgers_op* op, int first, int count, SweepPlan* out, cudaStream_t st) {
+    for (const auto& kv : op->plans)
+        if (kv.first.first == first && kv.first.second == count) {
+            *out = kv.second;
+            return AMDG_OK;
+        }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    AMDG_CK(cudaStreamIsCapturing(st, &cap));
+    AMDG_REQUIRE(cap == cudaStreamCaptureStatusNone, AMDG_ERR_STATE, "sweep plan built during stream capture");
+    op->plans.push_back({{first, count}, make_plan(op, first, count)});
+    *out = op->plans.back().second;
+    return upload_plans(op, st);
+}
+
+// The default sweeps run planned (kernels_plan.cu); an explicit sweep variant runs term by term
+// through the sweep trees, and so does one dimension, where every term is a single sweep.
+bool planned(const amdg_burgers_op* op) { return op->sweep_variant < 0 && op->grid->host.dim > 1; }
+
+// The terms [first, first + total) in the ranges that one launch sequence evaluates: all of them, or,
+// past the term budget, pieces of at most `chunk` terms of one group each, so that a group's sums do
+// not depend on what is evaluated beside it.
+std::vector<std::pair<int, int>> term_ranges(const amdg_burgers_op* op, int first, int total) {
+    std::vector<std::pair<int, int>> out;
+    if (total <= op->chunk) {
+        if (total > 0) out.push_back({first, total});
+        return out;
+    }
+    const int end = first + total;
+    for (int i = first; i < end;) {
+        int j = i;
+        while (j < end && j - i < op->chunk && op->terms[size_t(j)].grp == op->terms[size_t(i)].grp) ++j;
+        out.push_back({i, j - i});
+        i = j;
+    }
+    return out;
+}
+
 // the trees of every term range the right-hand side launches with the current chunk size, so a
 // step captured as a graph finds them all
 amdg_status prepare_trees(amdg_burgers_op* op, cudaStream_t st) {
     SweepTree t;
+    SweepPlan p;
     auto chunks = [&](int first, int total) -> amdg_status {
+        if (planned(op)) {
+            for (const auto& r : term_ranges(op, first, total))
+                if (amdg_status s = sweep_plan(op, r.first, r.second, &p, st); s != AMDG_OK) return s;
+            return AMDG_OK;
+        }
         for (int c0 = 0; c0 < total; c0 += op->chunk)
             if (amdg_status s = sweep_tree(op, first + c0, std::min(op->chunk, total - c0), &t, st); s != AMDG_OK) return s;
         return AMDG_OK;
@@ -290,8 +374,12 @@ amdg_status prepare_trees(amdg_burgers_op* op, cudaStream_t st) {
     amdg_status s;
     if (op->kind == 1) {
         const int G = int(op->sched_dims.size());
-        for (int f = 0; f <= dim; ++f)
-            if ((s = chunks(f * G, G)) != AMDG_OK) return s;
+        if (planned(op) && op->n_pv_terms <= op->chunk) {
+            if ((s = chunks(0, op->n_pv_terms)) != AMDG_OK) return s;
+        } else {
+            for (int f = 0; f <= dim; ++f)
+                if ((s = chunks(f * G, G)) != AMDG_OK) return s;
+        }
         if ((s = chunks(nterms - dim, dim)) != AMDG_OK) return s;
     } else if ((s = chunks(0, op->n_pv_terms)) != AMDG_OK) {
         return s;
@@ -358,6 +446,54 @@ amdg_status run_terms(amdg_burgers_op* op, const Mats<T>& m, int first, int coun
     return AMDG_OK;
 }
 
+// The planned sweeps of terms [first, first + count), the last one ending in `o`.
+template <typename T>
+amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count, int n_in, int n_out,
+                     const T* const* src, int nsrc, const T* pen_in, const PlanOut& o, cudaStream_t st) {
+    const amdg_grid* g = op->grid;
+    const int dim = g->host.dim;
+    const int64_t E = g->host.num_elements;
+    SweepPlan plan;
+    if (amdg_status s = sweep_plan(op, first, count, &plan, st); s != AMDG_OK) return s;
+    PlanArgs<T> a{};
+    a.dim = dim;
+    a.n1 = op->n1;
+    a.np = g->host.k + 1;
+    a.num_elements = E;
+    a.n_in = n_in;
+    a.n_out = n_out;
+    a.products = op->d_plan_products;
+    a.max_products = plan.max_products;
+    for (int i = 0; i < kNumLagrMats; ++i) a.mats[i] = m.m[i];
+    a.rows = static_cast<const RowRec*>(op->d_rows);
+    a.vol_nbr = reinterpret_cast<const int2*>(op->d_vol_nbr);
+    a.flx_nbr = reinterpret_cast<const int2*>(op->d_flx_nbr);
+    for (int i = 0; i < nsrc && i < kMaxTermSources; ++i) a.src[i] = src[i];
+    a.pen_in = pen_in;
+    a.long_count = op->d_long;
+    a.long_rows = op->d_long + kMaxDim;
+    a.long_stride = op->long_stride;
+    const T* cur = nullptr;
+    for (int j = 0; j < dim; ++j) {
+        a.first_sweep = j == 0;
+        a.in = cur;
+        a.in_slice = j == 0 ? 0 : E * ipow(n_out, j) * ipow(n_in, dim - j);
+        a.out_block = ipow(n_out, j + 1) * ipow(n_in, dim - j - 1);
+        a.nodes = op->d_plan_nodes + plan.offset[j];
+        a.num_nodes = plan.count[j];
+        if (a.num_nodes == 0) continue;  // only penalty terms: a single (last) sweep
+        if (j == dim - 1) {
+            AMDG_CK(launch_plan_out<T>(a, o, st));
+        } else {
+            a.out = static_cast<T*>(j % 2 == 0 ? op->w_s0 : op->w_s1);
+            AMDG_CK(launch_plan_sweep<T>(a, st));
+            cur = a.out;
+        }
+        op->grid->ctx->launches++;
+    }
+    return AMDG_OK;
+}
+
 // u_h at the interpolation points (FP64 or FP32 arithmetic): into up, or, when
 // fp is given, f(u) = u^2/2 at the points into fp
 template <typename T>
@@ -367,7 +503,20 @@ amdg_status eval_point_values(amdg_burgers_op* op, const Mats<T>& m, const T* u,
     const bool herm = op->kind == 3;  // the Hermite flux needs the slopes too: applied after the sum
     T* slots = static_cast<T*>(op->w_slots);
     const T* src[1] = {u};
-    for (int c0 = 0; c0 < op->n_pv_terms; c0 += op->chunk) {
+    if (planned(op)) {
+        const auto ranges = term_ranges(op, 0, op->n_pv_terms);
+        for (size_t i = 0; i < ranges.size(); ++i) {
+            PlanOut o{};
+            o.mode = (i + 1 == ranges.size() && fp && !herm) ? kEpiFlux : kEpiPoints;
+            o.first = i == 0 ? 1 : 0;
+            o.acc = up;
+            o.out[0] = fp;
+            if (amdg_status r = run_plan<T>(op, m, ranges[i].first, ranges[i].second, np, op->p1, src, 1, nullptr, o, st);
+                r != AMDG_OK)
+                return r;
+        }
+    }
+    for (int c0 = 0; !planned(op) && c0 < op->n_pv_terms; c0 += op->chunk) {
         const int cnt = std::min(op->chunk, op->n_pv_terms - c0);
         if (amdg_status r = run_terms<T>(op, m, c0, cnt, np, op->p1, src, 1, nullptr, slots, st); r != AMDG_OK) return r;
         const bool last = c0 + cnt == op->n_pv_terms;
@@ -392,7 +541,21 @@ amdg_status eval_point_values_df(amdg_burgers_op* op, const double* u, double* u
     op->grid->ctx->launches++;
     float2* slots = static_cast<float2*>(op->w_slots);
     const float2* src[1] = {udf};
-    for (int c0 = 0; c0 < op->n_pv_terms; c0 += op->chunk) {
+    if (planned(op)) {
+        const auto ranges = term_ranges(op, 0, op->n_pv_terms);
+        for (size_t i = 0; i < ranges.size(); ++i) {
+            PlanOut o{};
+            o.mode = (i + 1 == ranges.size() && fp && op->kind != 3) ? kEpiFlux : kEpiPoints;
+            o.first = i == 0 ? 1 : 0;
+            o.acc = up;
+            o.out[0] = fp;
+            if (amdg_status r = run_plan<float2>(op, mats_df(op), ranges[i].first, ranges[i].second, np, op->p1, src, 1,
+                                                 nullptr, o, st);
+                r != AMDG_OK)
+                return r;
+        }
+    }
+    for (int c0 = 0; !planned(op) && c0 < op->n_pv_terms; c0 += op->chunk) {
         const int cnt = std::min(op->chunk, op->n_pv_terms - c0);
         if (amdg_status r = run_terms<float2>(op, mats_df(op), c0, cnt, np, op->p1, src, 1, nullptr, slots, st);
             r != AMDG_OK)
@@ -450,6 +613,21 @@ template <typename T>
 amdg_status eval_term_range(amdg_burgers_op* op, const Mats<T>& m, int first, int total, const T* const* src, int nsrc,
                             const T* u, double* rhs, StageOut so, cudaStream_t st, bool accumulate = false) {
     const int np = op->grid->host.k + 1;
+    if (planned(op)) {
+        const auto ranges = term_ranges(op, first, total);
+        for (size_t i = 0; i < ranges.size(); ++i) {
+            PlanOut o{};
+            o.mode = kEpiRhs;
+            o.first = (i == 0 && !accumulate) ? 1 : 0;
+            o.last = i + 1 == ranges.size() ? 1 : 0;
+            o.acc = rhs;
+            o.so = so;
+            if (amdg_status r = run_plan<T>(op, m, ranges[i].first, ranges[i].second, op->p1, np, src, nsrc, u, o, st);
+                r != AMDG_OK)
+                return r;
+        }
+        return AMDG_OK;
+    }
     T* slots = static_cast<T*>(op->w_slots);
     for (int c0 = 0; c0 < total; c0 += op->chunk) {
         const int cnt = std::min(op->chunk, total - c0);
@@ -507,7 +685,43 @@ amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, c
         if constexpr (df) return mats_df(op);
         else return mats64(op);
     }();
-    for (int f = f_first; f <= (f_last < 0 ? dim : f_last); ++f) {
+    if (f_last < 0) f_last = dim;
+    if (planned(op)) {
+        const int first = f_first * G, total = (f_last - f_first + 1) * G;
+        if (total <= op->chunk) {  // every field in one sequence of sweeps, K applied in the last
+            PlanOut o{};
+            o.mode = kEpiCoef;
+            for (int f = f_first; f <= f_last; ++f) o.out[f - f_first] = fields + size_t(f) * stride;
+            o.order = g->d_order;
+            o.sines = op->d_sines;
+            o.amp = op->amp;
+            if (amdg_status r = run_plan<Tp>(op, m, first, total, np, op->p1, src, 1, nullptr, o, st); r != AMDG_OK)
+                return r;
+        } else {
+            for (int f = f_first; f <= f_last; ++f) {
+                double* acc = static_cast<double*>(op->w_up);
+                const auto ranges = term_ranges(op, f * G, G);
+                for (size_t i = 0; i < ranges.size(); ++i) {
+                    PlanOut o{};
+                    o.mode = kEpiPoints;
+                    o.first = i == 0 ? 1 : 0;
+                    o.acc = acc;
+                    if (amdg_status r = run_plan<Tp>(op, m, ranges[i].first, ranges[i].second, np, op->p1, src, 1,
+                                                     nullptr, o, st);
+                        r != AMDG_OK)
+                        return r;
+                }
+                AMDG_CK(launch_reduce_points_coef(acc, 1, E, dim, op->p1, g->d_order, op->d_pts, op->amp,
+                                                  fields + size_t(f) * stride, st));
+                op->grid->ctx->launches++;
+            }
+        }
+        for (int f = f_first; f <= f_last; ++f)
+            if (amdg_status r = eval_surplus<double, To>(op, fields + size_t(f) * stride, fucoe[f], st); r != AMDG_OK)
+                return r;
+        return AMDG_OK;
+    }
+    for (int f = f_first; f <= f_last; ++f) {
         double* kp = fields + size_t(f) * stride;  // K times the point values of field f
         double* acc = static_cast<double*>(op->w_up);
         for (int c0 = 0; c0 < G; c0 += op->chunk) {
@@ -629,6 +843,14 @@ amdg_status reserve_grow(amdg_burgers_op* op, T** p, size_t bytes) {
     return AMDG_OK;
 }
 
+// row records and long-row lists for the current element set
+amdg_status reserve_rows(amdg_burgers_op* op) {
+    const int64_t E = op->grid->host.num_elements, dim = op->grid->host.dim;
+    op->long_stride = E;
+    if (amdg_status s = reserve_grow(op, &op->d_rows, size_t(E * dim) * sizeof(RowRec)); s != AMDG_OK) return s;
+    return reserve_grow(op, &op->d_long, size_t(kMaxDim + E * dim) * sizeof(int32_t));
+}
+
 // The neighbour lists and surplus ancestors built on the device from the grid's keys
 // (csrc/adapt_device.cu), into arrays sized by the bounds of the element set's level sums.
 amdg_status device_topology(amdg_burgers_op* op, cudaStream_t st) {
@@ -645,7 +867,8 @@ amdg_status device_topology(amdg_burgers_op* op, cudaStream_t st) {
         (s = reserve_grow(op, &op->d_topo_cnt, size_t(2 * (rows + 1)) * sizeof(int32_t))) != AMDG_OK ||
         (s = reserve_grow(op, &op->d_vol_nbr, size_t(2 * vb) * sizeof(int32_t))) != AMDG_OK ||
         (s = reserve_grow(op, &op->d_flx_nbr, size_t(2 * fb) * sizeof(int32_t))) != AMDG_OK ||
-        (s = reserve_grow(op, &op->d_anc, size_t(rows) * op->p1 * sizeof(int32_t))) != AMDG_OK)
+        (s = reserve_grow(op, &op->d_anc, size_t(rows) * op->p1 * sizeof(int32_t))) != AMDG_OK ||
+        (s = reserve_rows(op)) != AMDG_OK)
         return s;
     if (!op->d_anc_order) {
         std::vector<int32_t> ao = op->anc_order;
@@ -656,7 +879,8 @@ amdg_status device_topology(amdg_burgers_op* op, cudaStream_t st) {
     const size_t vcap = op->dev_cap[static_cast<const void*>(&op->d_vol_nbr)] / (2 * sizeof(int32_t));
     const size_t fcap = op->dev_cap[static_cast<const void*>(&op->d_flx_nbr)] / (2 * sizeof(int32_t));
     DeviceTopoOut out{op->d_vol_ptr, op->d_vol_nbr, op->d_vol_split, op->d_flx_ptr, op->d_flx_nbr, op->d_flx_split,
-                      op->d_anc, int64_t(vcap), int64_t(fcap), op->d_anc_order, op->p1, err};
+                      op->d_anc, int64_t(vcap), int64_t(fcap), op->d_anc_order, op->p1, err,
+                      op->d_rows, op->d_long, op->d_long + kMaxDim, op->long_stride};
     if ((s = device_transform_topology(g, out, op->d_topo_cnt, st)) != AMDG_OK) return s;
     // a set that came from the host may have holes: report them now (sets the device refine and
     // coarsen produce are hole-free; their build errors surface at the next element-set change)
@@ -697,8 +921,13 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
             (s = upload_grow(op, &op->d_flx_nbr, topo.flx_nbr, st)) != AMDG_OK ||
             (s = upload_grow(op, &op->d_anc, anc, st)) != AMDG_OK ||
             (s = upload_grow(op, &op->d_vol_split, topo.vol_split, st)) != AMDG_OK ||
-            (s = upload_grow(op, &op->d_flx_split, topo.flx_split, st)) != AMDG_OK)
+            (s = upload_grow(op, &op->d_flx_split, topo.flx_split, st)) != AMDG_OK || (s = reserve_rows(op)) != AMDG_OK)
             return s;
+        AMDG_CK(cudaMemsetAsync(op->d_long, 0, kMaxDim * sizeof(int32_t), st));
+        AMDG_CK(launch_pack_rows(op->d_vol_ptr, op->d_vol_split, op->d_flx_ptr, op->d_flx_split, g->d_order,
+                                 g->host.num_elements, g->host.dim, static_cast<RowRec*>(op->d_rows), op->d_long,
+                                 op->d_long + kMaxDim, op->long_stride, st));
+        g->ctx->launches++;
         // the host vectors above are released on return: wait for their copies
         AMDG_CK(cudaStreamSynchronize(st));
     }
@@ -706,10 +935,10 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
     if (E > op->capacity) {
         const int64_t cap = E + E / 2 + 16;
         void* bufs[] = {op->w_up, op->w_fu, op->w_a, op->w_b, op->w_u, op->w_s0, op->w_s1, op->w_slots,
-                        op->d_u1, op->d_rhs64, op->d_pred, op->w_fields, op->d_v1, op->d_su, op->d_sv};
+                        op->d_u1, op->d_u2, op->d_rhs64, op->d_pred, op->w_fields, op->d_v1, op->d_su, op->d_sv};
         for (void* p : bufs) cudaFree(p);
         op->w_up = op->w_fu = op->w_a = op->w_b = op->w_u = op->w_s0 = op->w_s1 = op->w_slots = op->w_fields = nullptr;
-        op->d_u1 = op->d_rhs64 = op->d_pred = op->d_v1 = op->d_su = op->d_sv = nullptr;
+        op->d_u1 = op->d_u2 = op->d_rhs64 = op->d_pred = op->d_v1 = op->d_su = op->d_sv = nullptr;
         op->capacity = 0;
         const size_t work = size_t(cap) * op->points * sizeof(double);
         const size_t vec = size_t(cap) * g->block * sizeof(double);
@@ -723,6 +952,7 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
             (s = alloc_bytes(&op->w_u, vec)) != AMDG_OK || (s = alloc_bytes(&op->w_s0, slices)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_s1, slices)) != AMDG_OK || (s = alloc_bytes(&op->w_slots, slices)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_u1), vec)) != AMDG_OK ||
+            (s = alloc_bytes(reinterpret_cast<void**>(&op->d_u2), vec)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_rhs64), vec)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_pred), vec)) != AMDG_OK)
             return s;
@@ -835,13 +1065,20 @@ static amdg_status lagr_create(amdg_grid* g, int kind, const double* alpha, doub
     transform_schedule(dim, &op->sched_dims, &op->sched_lu);
     build_terms(op);
     amdg_status s;
+    auto point_sines = [&]() -> amdg_status {
+        if (amdg_status r = alloc_bytes(reinterpret_cast<void**>(&op->d_sines), t.pts.size() * sizeof(double)); r != AMDG_OK)
+            return r;
+        AMDG_CK(launch_point_sines(op->d_pts, op->d_sines, int(t.pts.size()), stream_of(op)));
+        g->ctx->launches++;
+        return AMDG_OK;
+    };
     if ((s = upload_both(&op->d_a2p, &op->f_a2p, t.a2p)) != AMDG_OK || (s = upload_both(&op->d_lv, &op->f_lv, t.lv)) != AMDG_OK ||
         (s = upload_both(&op->d_lvx, &op->f_lvx, t.lvx)) != AMDG_OK ||
         (s = upload_both(&op->d_lflx, &op->f_lflx, t.lflx)) != AMDG_OK ||
         (s = upload_both(&op->d_ajump, &op->f_ajump, t.ajump)) != AMDG_OK ||
         (kind == 1 && ((s = upload_both(&op->d_a2pd, &op->f_a2pd, t.a2pd)) != AMDG_OK ||
                        (s = upload_both(&op->d_ljv, &op->f_ljv, t.ljv)) != AMDG_OK ||
-                       (s = upload_vec(&op->d_pts, t.pts)) != AMDG_OK)) ||
+                       (s = upload_vec(&op->d_pts, t.pts)) != AMDG_OK || (s = point_sines()) != AMDG_OK)) ||
         (s = upload_df(&op->df_a2p, t.a2p)) != AMDG_OK || (kind == 1 && (s = upload_df(&op->df_a2pd, t.a2pd)) != AMDG_OK) ||
         (s = upload_vec(&op->d_anc_point, t.anc_point)) != AMDG_OK || (s = upload_vec(&op->d_anc_rank, t.anc_rank)) != AMDG_OK ||
         (s = upload_vec(&op->d_terms, op->terms)) != AMDG_OK || (s = burgers_sync(op)) != AMDG_OK) {
@@ -877,7 +1114,8 @@ amdg_status amdg_burgers_destroy(amdg_burgers_op* op) {
                     op->d_pg,
                     op->d_feat, op->d_prob, op->d_a2pd, op->d_ljv, op->d_pts, op->f_a2pd, op->f_ljv,
                     op->w_fields, op->d_v1, op->d_su, op->d_sv, op->df_a2p, op->df_a2pd,
-                    op->d_anc_order, op->d_topo_cnt, op->d_cls, op->d_nodes};
+                    op->d_anc_order, op->d_topo_cnt, op->d_cls, op->d_nodes, op->d_plan_nodes, op->d_plan_products,
+                    op->d_rows, op->d_long, op->d_sines};
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(op->h_cls);
     delete op;
@@ -918,14 +1156,18 @@ amdg_status amdg_burgers_work(amdg_burgers_op* op, double* flops, double* transf
             cnt[t][f][1] += ptr[f][r + 1] - ptr[f][r];
             cnt[t][f][2] += split[f][r] - ptr[f][r];      // "U": coarser or equal
         }
-    // the sweeps one right-hand side runs: the nodes of the sweep trees of its term ranges
+    // the sweeps one right-hand side runs: the products of its plans, or the nodes of its sweep trees
     double fl = 0.0, pairs = 0.0;
     std::vector<std::pair<int, int>> ranges;
     auto chunks = [&](int first, int total) {
+        if (planned(op)) {
+            for (const auto& r : term_ranges(op, first, total)) ranges.push_back(r);
+            return;
+        }
         for (int c0 = 0; c0 < total; c0 += op->chunk) ranges.push_back({first + c0, std::min(op->chunk, total - c0)});
     };
     const int nterms = int(op->terms.size());
-    if (op->kind == 1) {
+    if (op->kind == 1 && !(planned(op) && op->n_pv_terms <= op->chunk)) {
         const int G = int(op->sched_dims.size());
         for (int f = 0; f <= dim; ++f) chunks(f * G, G);
     } else {
@@ -933,22 +1175,34 @@ amdg_status amdg_burgers_work(amdg_burgers_op* op, double* flops, double* transf
     }
     chunks(op->n_pv_terms, nterms - op->n_pv_terms);
     for (const auto& r : ranges) {
-        SweepTree tree;
-        if (amdg_status s = sweep_tree(op, r.first, r.second, &tree, stream_of(op)); s != AMDG_OK) return s;
         const bool pv = r.first < op->n_pv_terms;
         const int n_in = pv ? np : p1, n_out = pv ? p1 : np;
+        // one transform along t of sweep j (j < 0: the penalty, a full transform on the flx sets)
+        auto add = [&](int j, int t, int flx, int lu) {
+            const double c = cnt[t][flx][lu];
+            fl += j < 0 ? 2.0 * np * ipow(np, dim) * c : 2.0 * n_in * ipow(n_out, j + 1) * ipow(n_in, dim - j - 1) * c;
+            pairs += c;
+        };
+        if (planned(op)) {
+            SweepPlan plan;
+            if (amdg_status s = sweep_plan(op, r.first, r.second, &plan, stream_of(op)); s != AMDG_OK) return s;
+            for (int j = 0; j < dim; ++j)
+                for (int k = 0; k < plan.count[j]; ++k) {
+                    const PlanNode& n = op->plan_nodes[size_t(plan.offset[j] + k)];
+                    for (int q = 0; q < n.count; ++q) {
+                        const PlanProduct& p = op->plan_products[size_t(n.first + q)];
+                        add(p.in < 0 ? -1 : j, p.t, p.flx, p.lu);
+                    }
+                }
+            continue;
+        }
+        SweepTree tree;
+        if (amdg_status s = sweep_tree(op, r.first, r.second, &tree, stream_of(op)); s != AMDG_OK) return s;
         for (int j = 0; j < dim; ++j)
             for (int k = 0; k < tree.count[j]; ++k) {
                 const PartialSum& D = op->nodes[size_t(tree.offset[j] + k)];
-                if (D.kind == 1) {  // the penalty: one full transform along dims[0] on the flx sets
-                    const double c = cnt[D.dims[0]][1][1];
-                    fl += 2.0 * np * ipow(np, dim) * c;
-                    pairs += c;
-                    continue;
-                }
-                const double c = cnt[D.dims[j]][D.flx[j]][D.lu[j]];
-                fl += 2.0 * n_in * ipow(n_out, j + 1) * ipow(n_in, dim - j - 1) * c;
-                pairs += c;
+                if (D.kind == 1) add(-1, D.dims[0], 1, 1);
+                else add(j, D.dims[j], D.flx[j], D.lu[j]);
             }
     }
     // hierarchical surplus passes (one field for Burgers, dim + 1 for the wave operator)
@@ -962,6 +1216,7 @@ amdg_status amdg_burgers_set_sweep_variant(amdg_burgers_op* op, int variant) {
     AMDG_REQUIRE(op && variant >= -1 && variant <= 4, AMDG_ERR_ARG, "variant must be -1 .. 4");
     op->sweep_variant = variant;
     op->graph_version = -1;  // a captured step launched the other kernel
+    op->built_version = -1;  // the next call prepares the other kernels' trees or plans
     return AMDG_OK;
 }
 
@@ -1082,16 +1337,15 @@ amdg_status amdg_burgers_rk3_steps(amdg_burgers_op* op, double dt, int nsteps, a
     PhaseTimer timer(g->ctx, AMDG_PHASE_RK3);
     cudaStream_t st = stream_of(op);
     if (nsteps == 0) return AMDG_OK;
-    const size_t bytes = size_t(g->dof) * sizeof(double);
-    // one step: ucoe is updated in place per stage, ucoe_tn holds u^n (RK3SSP::step_stage)
+    // one step: u^n stays in the grid's coefficients until the last stage writes them; a stage's output
+    // is another vector than its input, which the last sweep reads at neighbouring elements
     auto step = [&]() -> amdg_status {
-        AMDG_CK(cudaMemcpyAsync(op->d_u1, g->d_u, bytes, cudaMemcpyDeviceToDevice, st));
+        double* const in[3] = {g->d_u, op->d_u1, op->d_u2};
+        double* const out[3] = {op->d_u1, op->d_u2, g->d_u};
         for (int stage = 0; stage < 3; ++stage) {
-            // the last reduction applies the stage update in place (u1 is the stage input)
-            const StageOut so{1, stage_coef(stage, dt), g->d_u, op->d_u1, op->d_u1};
-            if (amdg_status r = eval_rhs(op, op->d_u1, op->d_rhs64, prec, so); r != AMDG_OK) return r;
+            const StageOut so{1, stage_coef(stage, dt), g->d_u, in[stage], out[stage]};
+            if (amdg_status r = eval_rhs(op, in[stage], op->d_rhs64, prec, so); r != AMDG_OK) return r;
         }
-        AMDG_CK(cudaMemcpyAsync(g->d_u, op->d_u1, bytes, cudaMemcpyDeviceToDevice, st));
         return AMDG_OK;
     };
     op->rhs_evaluations += 3 * int64_t(nsteps);

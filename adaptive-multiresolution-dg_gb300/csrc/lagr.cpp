@@ -371,6 +371,136 @@ SweepTree build_sweep_tree(const std::vector<PartialSum>& terms, int first, int 
     return tree;
 }
 
+namespace {
+
+// Builds the nodes of one plan from the last sweep down.
+struct PlanBuilder {
+    const std::vector<PartialSum>& terms;
+    int dim, n_in, n_out;
+    std::vector<std::vector<std::vector<PlanProduct>>> products;    // per sweep and node
+
+    static bool same_transform(const PartialSum& a, const PartialSum& b, int j) {
+        return a.dims[j] == b.dims[j] && a.lu[j] == b.lu[j] && a.mat[j] == b.mat[j] && a.flx[j] == b.flx[j];
+    }
+    static bool same_product(const PlanProduct& a, const PlanProduct& b) {
+        return a.in == b.in && a.t == b.t && a.lu == b.lu && a.flx == b.flx && a.mat == b.mat && a.coef == b.coef;
+    }
+    // sweep j of term t (its input block has the dimensions of sweeps 0 .. j - 1 transformed)
+    PlanProduct product(const PartialSum& t, int j) const {
+        PlanProduct p{};
+        p.t = t.dims[j];
+        p.lu = t.lu[j];
+        p.flx = t.flx[j];
+        p.mat = t.mat[j];
+        p.stride = 1;
+        p.in_block = 1;
+        for (int d = 0; d < dim; ++d) {
+            bool done = false;
+            for (int q = 0; q < j; ++q) done = done || t.dims[q] == d;
+            const int n = done ? n_out : n_in;
+            p.in_block *= n;
+            if (d > p.t) p.stride *= n;
+        }
+        p.coef = 1.0;
+        return p;
+    }
+    // the products of the sum over `set` of sweeps 0 .. j of its terms; a term's coefficient scales
+    // its last sweep
+    std::vector<PlanProduct> sum_of(const std::vector<int>& set, int j) {
+        std::vector<std::vector<int>> groups;
+        for (int i : set) {
+            const PartialSum& t = terms[size_t(i)];
+            size_t k = 0;
+            for (; j > 0 && k < groups.size(); ++k) {
+                const PartialSum& o = terms[size_t(groups[k][0])];
+                if (same_transform(t, o, j) && (j < dim - 1 || t.coef == o.coef)) break;
+            }
+            if (j == 0 || k == groups.size()) groups.push_back({i});
+            else groups[k].push_back(i);
+        }
+        std::vector<PlanProduct> out;
+        for (const auto& g : groups) {
+            const PartialSum& t = terms[size_t(g[0])];
+            PlanProduct p = product(t, j);
+            p.in = j == 0 ? t.src : node_of(sum_of(g, j - 1), j - 1);
+            if (j == dim - 1) p.coef = t.coef;
+            out.push_back(p);
+        }
+        return out;
+    }
+    int node_of(const std::vector<PlanProduct>& p, int j) {
+        for (size_t k = 0; k < products[j].size(); ++k) {
+            bool same = products[j][k].size() == p.size();
+            for (size_t q = 0; same && q < p.size(); ++q) same = same_product(products[j][k][q], p[q]);
+            if (same) return int(k);
+        }
+        products[j].push_back(p);
+        return int(products[j].size()) - 1;
+    }
+};
+
+}  // namespace
+
+SweepPlan build_sweep_plan(const std::vector<PartialSum>& terms, int first, int count, int dim, int n_in, int n_out,
+                           int np, bool node_per_group, std::vector<PlanNode>* nodes,
+                           std::vector<PlanProduct>* products) {
+    PlanBuilder b{terms, dim, n_in, n_out, {}};
+    b.products.resize(size_t(dim));
+    // the last sweep: per group the products of its terms, in term order
+    std::vector<PlanProduct> last;
+    for (int i = first; i < first + count;) {
+        const int grp = terms[size_t(i)].grp;
+        std::vector<int> set;
+        std::vector<PlanProduct> pen;
+        for (; i < first + count && terms[size_t(i)].grp == grp; ++i) {
+            const PartialSum& t = terms[size_t(i)];
+            if (t.kind == 0) {
+                set.push_back(i);
+                continue;
+            }
+            PlanProduct p{};
+            p.in = -1;
+            p.t = t.dims[0];
+            p.lu = 1;
+            p.flx = 1;
+            p.mat = kMatAJump;
+            p.stride = 1;
+            p.in_block = 1;
+            for (int d = 0; d < dim; ++d) {
+                p.in_block *= np;
+                if (d > p.t) p.stride *= np;
+            }
+            p.coef = t.coef;
+            pen.push_back(p);
+        }
+        std::vector<PlanProduct> sum;
+        if (!set.empty()) sum = b.sum_of(set, dim - 1);
+        sum.insert(sum.end(), pen.begin(), pen.end());
+        last.insert(last.end(), sum.begin(), sum.end());
+        if (node_per_group || i == first + count) {
+            b.products[size_t(dim - 1)].push_back(last);
+            last.clear();
+        }
+    }
+    SweepPlan plan;
+    for (int j = 0; j < dim; ++j) {
+        plan.offset[j] = int(nodes->size());
+        plan.count[j] = int(b.products[size_t(j)].size());
+        for (const auto& list : b.products[size_t(j)]) {
+            PlanNode n{int32_t(products->size()), int32_t(list.size()), -1, 0};
+            for (const PlanProduct& p : list)
+                if (p.lu != 2) {
+                    n.long_dim = p.t;
+                    n.long_mask |= 1 << p.t;
+                }
+            nodes->push_back(n);
+            products->insert(products->end(), list.begin(), list.end());
+            if (j == dim - 1) plan.max_products = std::max(plan.max_products, int(list.size()));
+        }
+    }
+    return plan;
+}
+
 void transform_schedule(int dim, std::vector<std::vector<int>>* dim_order, std::vector<std::vector<int>>* lu) {
     // 2^(dim-1) partial sums; sum s: dimension d gets tag 2*bit_d(s) for d < dim-1
     // and tag 1 for the last, then dimensions are ordered by tag
