@@ -310,12 +310,12 @@ amdg_status rk3_steps_device(amdg_linear_op* op, double dt, int nsteps, amdg_pre
                 g->ctx->launches++;
             }
         }
-        // a copy wait that gave up leaves the state as it was: the merge runs only after the check
-        if (L.variant >= 2 && check)
-            if (amdg_status s = check_copy_waits(op); s != AMDG_OK) return s;
-        AMDG_CK(launch_merge(hi[0], lo[0], u, g->dof, st));
+        // a copy wait that gave up leaves the state as it was: the merge reads the error flag, and the
+        // check (which waits for the stream) follows it
+        const bool checked = L.variant >= 2 && check;
+        AMDG_CK(launch_merge(hi[0], lo[0], u, g->dof, st, checked ? op->d_err : nullptr));
         g->ctx->launches++;
-        return AMDG_OK;
+        return checked ? check_copy_waits(op) : AMDG_OK;
     }
     for (int s = 0; s < nsteps; ++s) {
         // u1 = u + dt L(u); u2 = 3/4 u + 1/4 (u1 + dt L(u1)); u = 1/3 u + 2/3 (u2 + dt L(u2))

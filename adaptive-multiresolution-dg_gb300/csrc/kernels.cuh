@@ -157,7 +157,8 @@ bool linear_col_supported(int dim, int np);
 bool linear_mma_supported(int dim, int np);
 // FP64 vector <-> FP32 (hi, lo) pairs
 cudaError_t launch_split(const double* in, float* hi, float* lo, int64_t n, cudaStream_t st);
-cudaError_t launch_merge(const float* hi, const float* lo, double* out, int64_t n, cudaStream_t st);
+cudaError_t launch_merge(const float* hi, const float* lo, double* out, int64_t n, cudaStream_t st,
+                         const int* err = nullptr);
 DFState df_stage(StageCoef rk);
 cudaError_t launch_to_float(const double* in, float* out, int64_t n, cudaStream_t st);
 cudaError_t launch_stage_update(const double* un, double* u, const double* rhs, int64_t n, StageCoef rk, cudaStream_t st);
