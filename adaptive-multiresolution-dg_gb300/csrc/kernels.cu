@@ -18,6 +18,7 @@
 
 #include "kernels.cuh"
 #include "df_arith.cuh"
+#include "launch.cuh"
 
 namespace amdg {
 
@@ -198,6 +199,192 @@ __global__ void __launch_bounds__(256) linear_col_kernel(const double* __restric
         out[gid] = v;
         if (shadow_out) shadow_out[gid] = float(v);
     }
+}
+
+// Variant 0 for FP32 grids that fill the device, NP outputs per thread: the same sums in the same order
+// as linear_apply_kernel (bitwise equal), but the NP outputs share the neighbour indices and, per
+// neighbour, either the operator column (their index along t is the same) or the input column (they
+// are that column).  k = 3: NP consecutive outputs, the inputs as 16-byte loads (blocks of 4^D floats
+// are aligned); else NP outputs B / NP apart (along the first dimension), each load of a warp
+// consecutive.  Per NP^2 multiply-adds 2 NP (k = 3) or NP^2 + NP loads instead of 2 NP^2: the
+// single-output kernel is bound by the load/store unit there.  Stage times: 6D N = 8 k = 2 1028 -> 567
+// us, 5D N = 8 k = 2 161 -> 103, 5D N = 5 k = 3 29.6 -> 26.8, 5D N = 6 k = 2 25.3 -> 21.4.
+template <int D, int NP>
+__global__ void __launch_bounds__(256) linear_multi_kernel(const double* __restrict__ us, const float* __restrict__ xs,
+                                                           const double* un, double* out, float* shadow_out,
+                                                           const int32_t* __restrict__ row_ptr,
+                                                           const int2* __restrict__ pairs,
+                                                           const float* __restrict__ blocks, int nblocks,
+                                                           int64_t num_elements, StageCoef rk, DFState df) {
+    constexpr int B = IPow<NP, D>::v, C = B / NP;
+    constexpr int BS = (NP * NP + 3) / 4 * 4;
+    constexpr bool CONSECUTIVE = NP == 4;
+    constexpr int kColumn = CONSECUTIVE ? D - 1 : 0;  // the dimension along which the outputs lie
+    const int64_t gid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (gid >= num_elements * C) return;
+    const int64_t e = gid / C;
+    const int c = int(gid - e * C);
+    float acc[NP];
+#pragma unroll
+    for (int r = 0; r < NP; ++r) acc[r] = 0.f;
+#pragma unroll
+    for (int t = 0; t < D; ++t) {
+        int stride = 1;
+#pragma unroll
+        for (int s = t + 1; s < D; ++s) stride *= NP;
+        const int first = CONSECUTIVE ? c * NP : c;
+        const int qt = t == kColumn ? 0 : (first / stride) % NP;
+        const int base = first - qt * stride;
+        const int beg = __ldg(row_ptr + e * D + t), end = __ldg(row_ptr + e * D + t + 1);
+        const float* bt = blocks + size_t(t) * nblocks * BS;
+        auto neighbour = [&](int2 pr) {
+            const float* x = xs + int64_t(pr.x) * B + base;
+            const float* m = bt + size_t(pr.y) * BS;
+            if (t == kColumn) {
+                const BlockRegs<float, BS> mv = load_block<BS>(m);
+                float xv[NP];
+                if constexpr (CONSECUTIVE) {
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(x));
+                    xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[NP - 1] = v.w;
+                } else {
+#pragma unroll
+                    for (int p = 0; p < NP; ++p) xv[p] = __ldg(x + p * C);
+                }
+#pragma unroll
+                for (int p = 0; p < NP; ++p)
+#pragma unroll
+                    for (int r = 0; r < NP; ++r) acc[r] = fmaf(mv.v[p * NP + r], xv[p], acc[r]);
+            } else {
+                float xv[NP][NP], mv[NP];
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    mv[p] = __ldg(m + p * NP + qt);
+                    if constexpr (CONSECUTIVE) {
+                        const float4 v = __ldg(reinterpret_cast<const float4*>(x + p * stride));
+                        xv[p][0] = v.x; xv[p][1] = v.y; xv[p][2] = v.z; xv[p][NP - 1] = v.w;
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < NP; ++r) xv[p][r] = __ldg(x + p * stride + r * C);
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < NP; ++p)
+#pragma unroll
+                    for (int r = 0; r < NP; ++r) acc[r] = fmaf(mv[p], xv[p][r], acc[r]);
+            }
+        };
+        int i = beg;
+        for (; i + 2 <= end; i += 2) {
+            const int2 a = __ldg(pairs + i), b = __ldg(pairs + i + 1);
+            neighbour(a);
+            neighbour(b);
+        }
+        if (i < end) neighbour(__ldg(pairs + i));
+    }
+#pragma unroll
+    for (int r = 0; r < NP; ++r) {
+        const int64_t o = e * B + (CONSECUTIVE ? c * NP + r : c + r * C);
+        if (df.out_hi) {
+            df_stage_update(df, o, acc[r]);
+            continue;
+        }
+        const double rhs = double(acc[r]);
+        const double v = rk.mode == 0 ? rhs : rk_combine(rk.a, un[o], rk.b, us[o], rk.dt, rhs);
+        out[o] = v;
+        if (shadow_out) shadow_out[o] = float(v);
+    }
+}
+
+// Variant 0 for grids of few outputs, bound by the latency of one output's chain.  Launched so that it
+// may begin before the previous kernel of the stream has ended (launch_after): the neighbour indices
+// and operator entries, which no stage writes, are read before the wait for that kernel, and the
+// inputs of AHEAD neighbours are then loaded together.
+//
+// FP64: W = 4 warps share 32 outputs, warp w taking the neighbours k = w, w + W, ... of each output's
+// lists (all dimensions in sequence), the parts added in warp order.  An FP64 instruction holds a
+// quarter of a multiprocessor for 64 cycles whatever the number of its lanes (measured), so a stage
+// of such a grid lasts as long as one warp's chain of multiply-adds, with most of the device idle;
+// this divides the chain.  FP32: one warp, the order of linear_apply_kernel (the same bits).
+// 2D N = 7 (5,184 outputs): FP64 stage 15.6 -> 5.0 us.
+template <int D, int NP, typename T, int W, int AHEAD>
+__global__ void __launch_bounds__(32 * W) linear_split_kernel(const T* xs, const double* us, const double* un, double* out,
+                                                              const int32_t* __restrict__ row_ptr,
+                                                              const int2* __restrict__ pairs,
+                                                              const T* __restrict__ blocks, int nblocks, int64_t total,
+                                                              StageCoef rk, DFState df) {
+    constexpr int B = IPow<NP, D>::v;
+    constexpr int BS = (NP * NP + 3) / 4 * 4;
+    __shared__ T part[W][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t gid = int64_t(blockIdx.x) * 32 + lane;
+    const bool live = gid < total;
+    const int64_t e = live ? gid / B : 0;
+    const int q = int(gid - e * B);
+    int row[D + 1];
+#pragma unroll
+    for (int t = 0; t <= D; ++t) row[t] = __ldg(row_ptr + e * D + t);
+    const int n = live ? row[D] - row[0] : 0;
+    // neighbour k of the sequence: its first input entry, their distance and the operator entries
+    struct Nbr {
+        int64_t x;
+        int stride;
+        const T* m;
+    };
+    auto nbr_of = [&](int k) {
+        int t = 0;
+#pragma unroll
+        for (int s = 1; s < D; ++s) t += row[0] + k >= row[s] ? 1 : 0;
+        int stride = 1;
+#pragma unroll
+        for (int s = 1; s < D; ++s) stride *= s > t ? NP : 1;
+        const int2 pr = __ldg(pairs + row[0] + k);
+        const int qt = (q / stride) % NP;
+        return Nbr{int64_t(pr.x) * B + q - qt * stride, stride, blocks + (size_t(t) * nblocks + pr.y) * BS + qt};
+    };
+    int64_t x[AHEAD];
+    int stride[AHEAD];
+    T m[AHEAD][NP];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+        const int k = w + j * W;
+        x[j] = 0;
+        stride[j] = 0;
+        if (k < n) {
+            const Nbr b = nbr_of(k);
+            x[j] = b.x;
+            stride[j] = b.stride;
+#pragma unroll
+            for (int p = 0; p < NP; ++p) m[j][p] = __ldg(b.m + p * NP);
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    T acc = T(0), xv[AHEAD][NP];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+        if (w + j * W < n)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) xv[j][p] = xs[x[j] + p * stride[j]];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+        if (w + j * W < n)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) acc = fma(m[j][p], xv[j][p], acc);
+    for (int k = w + AHEAD * W; k < n; k += W) {
+        const Nbr b = nbr_of(k);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) acc = fma(__ldg(b.m + p * NP), xs[b.x + p * b.stride], acc);
+    }
+    if constexpr (W > 1) {
+        part[w][lane] = acc;
+        __syncthreads();
+        if (w != 0) return;
+#pragma unroll
+        for (int s = 1; s < W; ++s) acc += part[s][lane];
+    }
+    if (!live) return;
+    if constexpr (std::is_same<T, float>::value) df_stage_update(df, gid, acc);
+    else out[gid] = rk.mode == 0 ? acc : rk_combine(rk.a, un[gid], rk.b, us[gid], rk.dt, acc);
 }
 
 template <int D, int NP, typename T, typename X>
@@ -865,6 +1052,9 @@ bool linear_col_supported(int dim, int np) {
     return B / np <= 256;
 }
 
+constexpr int kMultiThreads = 1280;
+constexpr int kSplitOutputs = 512;  // per multiprocessor
+
 template <int D, int NP, typename T, typename X>
 static cudaError_t launch_linear_t(const LinearLaunch& L, const T* blocks, const X* xs, StageCoef rk, cudaStream_t st) {
     constexpr int B = IPow<NP, D>::v;
@@ -877,6 +1067,31 @@ static cudaError_t launch_linear_t(const LinearLaunch& L, const T* blocks, const
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             sms = 152;
+    }
+    if constexpr (std::is_same<T, float>::value && std::is_same<X, float>::value && D >= 2 && NP >= 3) {
+        // the threads must still fill the device: at 5D N = 4 k = 3 (540 threads per multiprocessor)
+        // 13 us with one output per thread, 21 us with four; at 1,580 (5D N = 6 k = 2) 25 and 21
+        const bool aligned = NP != 4 || (reinterpret_cast<uintptr_t>(xs) & 15) == 0;
+        if (total / NP >= int64_t(kMultiThreads) * sms && aligned) {
+            linear_multi_kernel<D, NP><<<unsigned((total / NP + 255) / 256), 256, 0, st>>>(
+                L.us, xs, L.un, L.out, L.shadow_out, L.row_ptr, L.pairs, L.blocks32p, L.num_blocks, L.num_elements, rk, L.df);
+            return cudaGetLastError();
+        }
+    }
+    // measured to 300 outputs per multiprocessor, split against not: FP64 2D N = 9 k = 3 19.7 / 60 us, 3D
+    // N = 7 12.2 / 22.8, 4D N = 5 11.1 / 15.2; at 700 the FP64 pipe is busy either way
+    if (total <= int64_t(kSplitOutputs) * sms) {
+        const dim3 grid(unsigned((total + 31) / 32));
+        if constexpr (std::is_same<T, double>::value) {
+            if (!L.shadow_out)
+                return launch_after(linear_split_kernel<D, NP, double, 4, 6>, grid, 128, 0, st, L.us, L.us, L.un, L.out,
+                                    L.row_ptr, L.pairs, L.blocks64p, L.num_blocks, total, rk, L.df);
+        } else if constexpr (std::is_same<X, float>::value) {
+            // (k = 3: 28.9 us against 27.5 at 2D N = 9, the operands read ahead take too many registers)
+            if (L.df.out_hi && NP <= 3)
+                return launch_after(linear_split_kernel<D, NP, float, 1, 12>, grid, 32, 0, st, xs, L.us, L.un, L.out,
+                                    L.row_ptr, L.pairs, L.blocks32p, L.num_blocks, total, rk, L.df);
+        }
     }
     int threads = 256;
     while (threads > 32 && (total + threads - 1) / threads < 2 * int64_t(sms)) threads /= 2;
