@@ -357,8 +357,7 @@ __global__ void __launch_bounds__(32 * W) linear_split_kernel(const T* xs, const
             for (int p = 0; p < NP; ++p) m[j][p] = __ldg(b.m + p * NP);
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
     T acc = T(0), xv[AHEAD][NP];
 #pragma unroll
     for (int j = 0; j < AHEAD; ++j)

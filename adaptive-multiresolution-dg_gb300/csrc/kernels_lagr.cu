@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "kernels_lagr.cuh"
+#include "launch.cuh"
 #include "sweep_math.cuh"
 
 namespace amdg {
@@ -476,15 +477,18 @@ cudaError_t launch_reduce_rhs(const T* buf, int count, int64_t n, int first, int
 template cudaError_t launch_reduce_rhs<double>(const double*, int, int64_t, int, int, double*, StageOut, cudaStream_t);
 template cudaError_t launch_reduce_rhs<float>(const float*, int, int64_t, int, int, double*, StageOut, cudaStream_t);
 
+// The ancestors' addresses and weights, which no pass writes, are read before the wait for the previous
+// kernel (launch_after).
 template <typename Ti, typename To>
-__global__ void __launch_bounds__(256) surplus_pass_kernel(SurplusArgs<Ti> a, const Ti* __restrict__ in, To* __restrict__ out) {
+__global__ void __launch_bounds__(256) surplus_pass_kernel(SurplusArgs<Ti> a, const Ti* in, To* out) {
     const int64_t gid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t total = a.num_elements * a.points;
-    if (gid >= total) return;
-    const int64_t e = gid / a.points;
+    const bool inside = gid < total;
+    const int64_t e = inside ? gid / a.points : 0;
     const int p = int(gid - e * a.points);
-    Ti c = in[gid];
-    const int od = __ldg(a.order + e * a.dim + a.d);
+    const int od = inside ? __ldg(a.order + e * a.dim + a.d) : 0;
+    int64_t at[kMaxLagrPoints];
+    double w[kMaxLagrPoints];
     if (od != 0) {
         const int P1 = a.p1;
         const int pd = (p / a.stride) % P1;
@@ -492,13 +496,27 @@ __global__ void __launch_bounds__(256) surplus_pass_kernel(SurplusArgs<Ti> a, co
         const int32_t* anc = a.anc + (e * a.dim + a.d) * P1;
         // Hermite: the level-1 weights scaled to the element's level (a power of two, exact)
         const int lscale = a.herm ? (31 - __clz(od)) : 0;
-        for (int ic = 0; ic < P1; ++ic) {
+#pragma unroll
+        for (int ic = 0; ic < kMaxLagrPoints; ++ic) {
+            if (ic >= P1) break;
             const int s = __ldg(anc + ic);
             const int q = __ldg(a.anc_point + od * P1 + ic);
             const int r = __ldg(a.anc_rank + od * P1 + ic);
-            const double w = a.herm ? ldexp(a.weight[pd * P1 + r], lscale * (pd / 2 - r / 2)) : a.weight[pd * P1 + r];
-            c = fma(Ti(w), in[int64_t(s) * a.points + base + q * a.stride], c);
+            at[ic] = int64_t(s) * a.points + base + q * a.stride;
+            w[ic] = a.herm ? ldexp(a.weight[pd * P1 + r], lscale * (pd / 2 - r / 2)) : a.weight[pd * P1 + r];
         }
+    }
+    wait_for_previous();
+    if (!inside) return;
+    Ti c = in[gid];
+    if (od != 0) {
+        Ti v[kMaxLagrPoints];
+#pragma unroll
+        for (int ic = 0; ic < kMaxLagrPoints; ++ic)
+            if (ic < a.p1) v[ic] = in[at[ic]];
+#pragma unroll
+        for (int ic = 0; ic < kMaxLagrPoints; ++ic)
+            if (ic < a.p1) c = fma(Ti(w[ic]), v[ic], c);
     }
     out[gid] = To(c);
 }
@@ -507,8 +525,8 @@ template <typename Ti, typename To>
 cudaError_t launch_surplus_pass(const SurplusArgs<Ti>& a, const Ti* in, To* out, cudaStream_t st) {
     const int64_t total = a.num_elements * a.points;
     if (total == 0) return cudaSuccess;
-    surplus_pass_kernel<Ti, To><<<AMDG_EW_GRID(total), 0, st>>>(a, in, out);
-    return cudaGetLastError();
+    const int th = ew_threads(total);
+    return launch_after(surplus_pass_kernel<Ti, To>, dim3(unsigned((total + th - 1) / th)), unsigned(th), 0, st, a, in, out);
 }
 
 template cudaError_t launch_surplus_pass<double, double>(const SurplusArgs<double>&, const double*, double*, cudaStream_t);

@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "kernels_plan.cuh"
+#include "launch.cuh"
 #include "sweep_math.cuh"
 
 namespace amdg {
@@ -31,6 +32,8 @@ namespace {
 
 constexpr int kSweepCta = 128;    // middle sweeps
 constexpr int kOutCta = 256;      // largest CTA of the last sweep
+constexpr int64_t kSharedEntries = 8192;  // outputs of a sweep (elements x entries) up to which four lanes share one
+constexpr int kSharedPhases = 4;
 constexpr size_t kPartBytes = 32 * 1024;  // shared memory for the products' parts
 constexpr int kLongItems = 4;     // output entries of a long row's unit in the last sweep
 
@@ -99,14 +102,38 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
             x[j] = in + int64_t(nb[j].x) * f.in_block;
             mm[j] = m + size_t(nb[j].y) * f.mstep;
         }
-        acc = fibre_quad<NF>(x, mm, f.stride, NT, acc);
+        if constexpr (std::is_same<T, float>::value) {
+            // FP32: each neighbour's part by itself, then pairwise (fewer roundings on the long sum)
+            float xv[4][NF], mv[4][NF], part[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int k = 0; k < NF; ++k) {
+                    xv[j][k] = x[j][k * f.stride];
+                    mv[j][k] = __ldg(mm[j] + k * NT);
+                }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                part[j] = xv[j][0] * mv[j][0];
+#pragma unroll
+                for (int k = 1; k < NF; ++k) part[j] = fmaf(xv[j][k], mv[j][k], part[j]);
+            }
+            acc += (part[0] + part[1]) + (part[2] + part[3]);
+        } else {
+            acc = fibre_quad<NF>(x, mm, f.stride, NT, acc);
+        }
     }
     for (; i < f.end; i += P) {
         const int2 nb = __ldg(f.nbr + i);
         const T* x = in + int64_t(nb.x) * f.in_block;
         const T* mm = m + size_t(nb.y) * f.mstep;
+        T part;
+        if constexpr (std::is_same<T, float>::value) part = x[0] * __ldg(mm);
+        else part = madd(x[0], __ldg(mm), acc);
 #pragma unroll
-        for (int k = 0; k < NF; ++k) acc = madd(__ldg(x + k * f.stride), __ldg(mm + k * NT), acc);
+        for (int k = 1; k < NF; ++k) part = madd(x[k * f.stride], __ldg(mm + k * NT), part);
+        if constexpr (std::is_same<T, float>::value) acc += part;
+        else acc = part;
     }
     return times(acc, f.coef);
 }
@@ -151,13 +178,18 @@ __device__ __forceinline__ void fibre_column_n(const Fibre<T>& f, int c, T (&acc
             T xa[NF], xb[NF], ma[BS], mb[BS];
 #pragma unroll
             for (int k = 0; k < NF; ++k) {
-                xa[k] = __ldg(x0 + k * f.stride);
-                xb[k] = __ldg(x1 + k * f.stride);
+                xa[k] = x0[k * f.stride];
+                xb[k] = x1[k * f.stride];
             }
             load_block<T, BS>(f.m + size_t(nb[j].y) * f.mstep, ma);
             load_block<T, BS>(f.m + size_t(nb[j + 1].y) * f.mstep, mb);
-            add_part<T, NF, NT>(xa, ma, acc);
-            if (i + j + 1 < f.end) add_part<T, NF, NT>(xb, mb, acc);
+            T pair[NT];
+#pragma unroll
+            for (int q = 0; q < NT; ++q) set_zero(pair[q]);
+            add_part<T, NF, NT>(xa, ma, pair);
+            if (i + j + 1 < f.end) add_part<T, NF, NT>(xb, mb, pair);
+#pragma unroll
+            for (int q = 0; q < NT; ++q) acc[q] = add_t(acc[q], pair[q]);
         }
     }
 #pragma unroll
@@ -183,12 +215,12 @@ __device__ __forceinline__ bool long_row(const PlanArgs<T>& a, const PlanNode& n
     return false;
 }
 
-// sum over the kLongPhases lanes of an output (phase = lane % 8) in a fixed order
-template <typename T>
+// sum over the P lanes of an output (phase = lane % P) in a fixed order; whole warps
+template <int P, typename T>
 __device__ __forceinline__ T phase_sum(T v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int off = 1; off < kLongPhases; off *= 2) v = add_t(v, shfl_from(v, lane ^ off));
+    for (int off = 1; off < P; off *= 2) v = add_t(v, shfl_from(v, lane ^ off));
     return v;
 }
 
@@ -196,10 +228,19 @@ __device__ __forceinline__ T phase_sum(T v) {
 
 // CTAs of 128 threads in at most 64 registers, eight per multiprocessor, as the single-term sweep
 // kernel (kernels_lagr.cu) was measured best.
-template <typename T, int NF, int NT, bool COL>
+// P: lanes per output entry (not COL).  What the sweeps do not write -- nodes, products, row records --
+// is read before the wait for the previous kernel (launch_after).
+template <typename T, int NF, int NT, bool COL, int P>
 __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel(PlanArgs<T> a) {
     const PlanNode node = a.nodes[blockIdx.y];
     const PlanProduct* prods = a.products + node.first;
+    const int64_t r = (int64_t(blockIdx.x) * kSweepCta + threadIdx.x) / P;
+    const bool inside = !COL && r < a.num_elements * a.out_block;
+    const int64_t re = inside ? r / a.out_block : 0;
+    const bool mine = inside && !long_row(a, node, re);
+    Fibre<T> f0{};
+    if (mine) f0 = fibre_of<T, NF, NT>(a, prods[0], re);
+    wait_for_previous();
     T* out = a.out + int64_t(blockIdx.y) * a.num_elements * a.out_block;
     if (node.long_dim >= 0) {  // long rows: units of 16 output entries x 8 phases
         constexpr int kItems = kSweepCta / kLongPhases;
@@ -216,7 +257,7 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
                 T part;
                 set_zero(part);
                 if (idx < a.out_block) part = fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[p], e), idx, ph, kLongPhases);
-                sum = add_t(sum, phase_sum(part));
+                sum = add_t(sum, phase_sum<kLongPhases>(part));
             }
             if (ph == 0 && idx < a.out_block) out[e * a.out_block + idx] = sum;
         }
@@ -265,15 +306,16 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
                 if (!long_row(a, node, e0 + j / a.out_block)) out[e0 * a.out_block + j] = y[j];
         }
     } else {
-        const int64_t r = int64_t(blockIdx.x) * kSweepCta + threadIdx.x;
-        if (r >= a.num_elements * a.out_block) return;
-        const int64_t e = r / a.out_block;
-        const int item = int(r - e * a.out_block);
-        if (long_row(a, node, e)) return;
-        T sum = fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[0], e), item, 0, 1);
-        for (int p = 1; p < node.count; ++p)
-            sum = add_t(sum, fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[p], e), item, 0, 1));
-        out[r] = sum;
+        const int item = int(r - re * a.out_block), ph = threadIdx.x % P;
+        T sum;
+        set_zero(sum);
+        if (mine) {
+            sum = fibre_entry<T, NF, NT>(f0, item, ph, P);
+            for (int p = 1; p < node.count; ++p)
+                sum = add_t(sum, fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[p], re), item, ph, P));
+        }
+        sum = phase_sum<P>(sum);
+        if (mine && ph == 0) out[r] = sum;
     }
 }
 
@@ -319,7 +361,7 @@ __device__ __forceinline__ void plan_epilogue(const PlanArgs<T>& a, const PlanOu
 // list, one trip count, one branch.  (Lanes spread over the products of one entry instead took 140 us
 // against 47 us on the FP64 right-hand side of 1,696 3D elements: the FP64 pipe, at 87 %, spent
 // most of its slots on masked lanes.)
-template <typename T, int NF, int NT, bool COL>
+template <typename T, int NF, int NT, bool COL, int P>
 __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, PlanOut o, int G, int W) {
     const int field = blockIdx.y;
     const PlanNode node = a.nodes[field];
@@ -328,6 +370,32 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
     extern __shared__ __align__(16) unsigned char smem[];
     T* part = reinterpret_cast<T*>(smem);
     const int tid = threadIdx.x;
+    // the first task of the warp, its row read before the wait for the previous kernel
+    // W: output entries per element of this CTA's window of the blocks (all of them unless the blocks
+    // are large; COL: all)
+    const int w0 = int(blockIdx.z) * W;
+    const int items = COL ? a.out_block / NT : min(W, a.out_block - w0);
+    const int lanes = G * items * P, chunks = (lanes + 31) / 32;
+    const int64_t e0 = int64_t(blockIdx.x) * G;
+    struct Task {
+        int p, g, item;
+        int64_t e;
+        bool live;
+    };
+    auto task_of = [&](int task) {
+        Task k;
+        k.p = task / chunks;
+        const int l = ((task - k.p * chunks) * 32 + (tid & 31)) / P;
+        k.g = l / items;
+        k.item = l - k.g * items;
+        k.e = e0 + k.g;
+        k.live = task < np * chunks && k.g < G && k.e < a.num_elements && !long_row(a, node, k.e);
+        return k;
+    };
+    const Task first = task_of(tid >> 5);
+    Fibre<T> f0{};
+    if (first.live) f0 = fibre_of<T, NF, NT>(a, prods[first.p], first.e);
+    wait_for_previous();
     if (node.long_mask) {
         // elements with a long row in a dimension that a non-"U" product transforms: kLongItems output
         // entries x np products as slots of 8 phases
@@ -352,7 +420,7 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
                     set_zero(v);
                     if (k < total && idx < a.out_block)
                         v = fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[k / kLongItems], e), idx, ph, kLongPhases);
-                    v = phase_sum(v);
+                    v = phase_sum<kLongPhases>(v);
                     if (ph == 0 && k < total) part[k] = v;
                 }
                 __syncthreads();
@@ -363,28 +431,24 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
             first_unit += cnt;
         }
     }
-    // W: output entries per element of this CTA's window of the blocks (all of them unless the blocks
-    // are large; COL: all)
-    const int w0 = int(blockIdx.z) * W;
-    const int items = COL ? a.out_block / NT : min(W, a.out_block - w0);
-    const int lanes = G * items, chunks = (lanes + 31) / 32;
-    const int64_t e0 = int64_t(blockIdx.x) * G;
     for (int task = tid >> 5; task < np * chunks; task += blockDim.x >> 5) {
-        const int p = task / chunks;
-        const int l = (task - p * chunks) * 32 + (tid & 31);
-        const int g = l / items, item = l - g * items;
-        const int64_t e = e0 + g;
-        if (g >= G || e >= a.num_elements || long_row(a, node, e)) continue;
-        const Fibre<T> f = fibre_of<T, NF, NT>(a, prods[p], e);
-        T* y = part + (p * G + g) * W;
+        const bool again = task != (tid >> 5);
+        const Task k = again ? task_of(task) : first;
+        if (again && k.live) f0 = fibre_of<T, NF, NT>(a, prods[k.p], k.e);
+        T* y = part + (k.p * G + k.g) * W;
         if constexpr (COL) {
+            if (!k.live) continue;
             T acc[NT];
-            fibre_column<T, NF, NT>(f, item, acc);
-            y += (item / f.stride) * f.stride * NT + item % f.stride;
+            fibre_column<T, NF, NT>(f0, k.item, acc);
+            y += (k.item / f0.stride) * f0.stride * NT + k.item % f0.stride;
 #pragma unroll
-            for (int q = 0; q < NT; ++q) y[q * f.stride] = acc[q];
+            for (int q = 0; q < NT; ++q) y[q * f0.stride] = acc[q];
         } else {
-            y[item] = fibre_entry<T, NF, NT>(f, w0 + item, 0, 1);
+            T v;
+            set_zero(v);
+            if (k.live) v = fibre_entry<T, NF, NT>(f0, w0 + k.item, tid % P, P);
+            v = phase_sum<P>(v);
+            if (k.live && tid % P == 0) y[k.item] = v;
         }
     }
     __syncthreads();
@@ -405,24 +469,34 @@ bool plan_supported(int n_in, int n_out) {
 
 namespace {
 
+// lanes per output entry: on grids of few outputs a launch lasts as long as one thread's chain over its
+// rows, so four lanes share an entry.  Measured with the limit at 0 / 8 k / 24 k / 64 k outputs: adaptive
+// 2D Hermite step (190-390 elements) 514 / 436 / 433 / 434 us, adaptive 3D step (830-1,170 elements) 866 /
+// 867 / 884 / 1,116 us: beyond it the FP64 pipe is busy and the four parts' sums only add to its work.
+template <typename T>
+bool shared_entries(const PlanArgs<T>& a) {
+    return a.num_elements * a.out_block <= kSharedEntries;
+}
+
 template <typename T, int NF, int NT>
 cudaError_t sweep_nn(const PlanArgs<T>& a, cudaStream_t st) {
     // FP32: a thread per column (a third of the operand loads; FP64 and double-float sums are bound
     // by their arithmetic and keep a thread per entry), unless an element's columns exceed a CTA
     const int cols = a.out_block / NT;
-    if (std::is_same<T, float>::value && cols <= kSweepCta) {
+    const bool shared = shared_entries(a);
+    if (std::is_same<T, float>::value && cols <= kSweepCta && !shared) {
         const int G = kSweepCta / cols;
         const dim3 grid(unsigned((a.num_elements + G - 1) / G), unsigned(a.num_nodes));
-        plan_sweep_kernel<T, NF, NT, std::is_same<T, float>::value>
-            <<<grid, kSweepCta, size_t(G) * a.out_block * sizeof(T), st>>>(a);
-    } else {
-        const dim3 grid(unsigned((a.num_elements * a.out_block + kSweepCta - 1) / kSweepCta), unsigned(a.num_nodes));
-        plan_sweep_kernel<T, NF, NT, false><<<grid, kSweepCta, 0, st>>>(a);
+        return launch_after(plan_sweep_kernel<T, NF, NT, std::is_same<T, float>::value, 1>, grid, kSweepCta,
+                            size_t(G) * a.out_block * sizeof(T), st, a);
     }
-    return cudaGetLastError();
+    const int64_t threads = a.num_elements * a.out_block * (shared ? kSharedPhases : 1);
+    const dim3 grid(unsigned((threads + kSweepCta - 1) / kSweepCta), unsigned(a.num_nodes));
+    return launch_after(shared ? plan_sweep_kernel<T, NF, NT, false, kSharedPhases> : plan_sweep_kernel<T, NF, NT, false, 1>,
+                        grid, kSweepCta, 0, st, a);
 }
 
-template <typename T, int NF, int NT, bool COL>
+template <typename T, int NF, int NT, bool COL, int P>
 cudaError_t out_col(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
     // windows of the blocks whose parts take at most 32 KB of shared memory; of whole blocks, the
     // fewest elements per CTA that leave at most a quarter of the lanes idle; warps for the tasks, or
@@ -430,7 +504,7 @@ cudaError_t out_col(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
     const int np = a.max_products;
     const int most = int(kPartBytes / (sizeof(T) * size_t(np)));
     const int W = COL ? a.out_block : std::min(a.out_block, std::max(32, most / 32 * 32));
-    const int items = COL ? a.out_block / NT : W;
+    const int items = (COL ? a.out_block / NT : W) * P;
     int G = 1;
     while (G < 32 && W == a.out_block && (G + 1) * W <= most && 4 * G * items < 3 * (32 * ((G * items + 31) / 32))) ++G;
     const int tasks = np * ((G * items + 31) / 32);
@@ -439,16 +513,16 @@ cudaError_t out_col(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
     const dim3 grid(unsigned((a.num_elements + G - 1) / G), unsigned(a.num_nodes), unsigned((a.out_block + W - 1) / W));
     const size_t smem = sizeof(T) * size_t(np) * std::max(G * W, kLongItems);
     if (smem > 48 * 1024) return cudaErrorInvalidValue;
-    plan_out_kernel<T, NF, NT, COL><<<grid, threads, smem, st>>>(a, o, G, W);
-    return cudaGetLastError();
+    return launch_after(plan_out_kernel<T, NF, NT, COL, P>, grid, unsigned(threads), smem, st, a, o, G, W);
 }
 
 template <typename T, int NF, int NT>
 cudaError_t out_nn(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
+    if (shared_entries(a)) return out_col<T, NF, NT, false, kSharedPhases>(a, o, st);
     // FP32: a thread per column where an element's parts fit
     if constexpr (std::is_same<T, float>::value)
-        if (sizeof(T) * size_t(a.max_products) * a.out_block <= kPartBytes) return out_col<T, NF, NT, true>(a, o, st);
-    return out_col<T, NF, NT, false>(a, o, st);
+        if (sizeof(T) * size_t(a.max_products) * a.out_block <= kPartBytes) return out_col<T, NF, NT, true, 1>(a, o, st);
+    return out_col<T, NF, NT, false, 1>(a, o, st);
 }
 
 }  // namespace

@@ -27,4 +27,13 @@ cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size
     return cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
 }
 
+#ifdef __CUDACC__
+// wait until the previous kernel of the stream has ended and its writes are visible, then let the next
+// kernel begin
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 }  // namespace amdg

@@ -55,7 +55,8 @@ __device__ __forceinline__ double to_double(float v) { return double(v); }
 __device__ __forceinline__ double to_double(float2 v) { return double(v.x) + double(v.y); }
 
 // acc + sum over four neighbours j (in order) and k < NF of x[j][k*stride] * m[j][k*ncols],
-// all operands loaded before the first multiply-add
+// all operands loaded before the first multiply-add.  (The inputs x by plain loads: a kernel launched
+// ahead of its predecessor's end must not read what that one writes through the read-only path.)
 template <int NF, typename T>
 __device__ __forceinline__ T fibre_quad(const T* const* x, const T* const* m, int stride, int ncols, T acc) {
     T xv[4][NF], mv[4][NF];
@@ -63,7 +64,7 @@ __device__ __forceinline__ T fibre_quad(const T* const* x, const T* const* m, in
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
-            xv[j][k] = __ldg(x[j] + k * stride);
+            xv[j][k] = x[j][k * stride];
             mv[j][k] = __ldg(m[j] + size_t(k) * ncols);
         }
 #pragma unroll
