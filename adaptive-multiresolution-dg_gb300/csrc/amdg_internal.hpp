@@ -274,6 +274,8 @@ struct PlanProduct {
     int32_t in;
     int8_t t, lu, flx, mat;
     int32_t stride, in_block;  // of the input block: entries between indices along t, entries per element
+    uint32_t stride_inv;       // ceil(2^32 / stride) for divisions by multiplication, 0 for stride 1
+    int32_t scaled;            // coef is not 1
     double coef;
 };
 struct PlanNode {

@@ -51,10 +51,14 @@ amdg_status upload_vec(T** p, const std::vector<T>& host) {
     return AMDG_OK;
 }
 
-amdg_status upload_both(double** d, float** f, const std::vector<double>& host) {
+// a table of blocks of n entries, FP64 and FP32 (the FP32 blocks padded, table_stride<float>)
+amdg_status upload_both(double** d, float** f, const std::vector<double>& host, int n) {
     amdg_status s = upload_vec(d, host);
     if (s != AMDG_OK) return s;
-    std::vector<float> h32(host.begin(), host.end());
+    const size_t pad = size_t((n + 3) / 4 * 4), blocks = host.size() / size_t(n);
+    std::vector<float> h32(blocks * pad, 0.0f);
+    for (size_t b = 0; b < blocks; ++b)
+        for (int i = 0; i < n; ++i) h32[b * pad + i] = float(host[b * n + i]);
     return upload_vec(f, h32);
 }
 
@@ -572,13 +576,15 @@ amdg_status eval_point_values_df(amdg_burgers_op* op, const double* u, double* u
 }
 
 // interpolation coefficients from values at the points: dim surplus passes
-// (w_a / w_b as ping-pong buffers), the last one into `out` (type To)
+// (w_a / w_b as ping-pong buffers, of several fields the sweep buffers), the last one into `out` (type
+// To); the fields in_field / out_field entries apart
 template <typename T, typename To>
-amdg_status eval_surplus(amdg_burgers_op* op, const T* in, To* out, cudaStream_t st) {
+amdg_status eval_surplus(amdg_burgers_op* op, const T* in, To* out, cudaStream_t st, int fields = 1, int64_t in_field = 0,
+                         int64_t out_field = 0) {
     const amdg_grid* g = op->grid;
     const int dim = g->host.dim;
-    T* ta = static_cast<T*>(op->w_a);
-    T* tb = static_cast<T*>(op->w_b);
+    T* ta = static_cast<T*>(fields > 1 ? op->w_s0 : op->w_a);
+    T* tb = static_cast<T*>(fields > 1 ? op->w_s1 : op->w_b);
     SurplusArgs<T> a{};
     a.dim = dim;
     a.p1 = op->p1;
@@ -590,14 +596,19 @@ amdg_status eval_surplus(amdg_burgers_op* op, const T* in, To* out, cudaStream_t
     a.anc_rank = op->d_anc_rank;
     for (int i = 0; i < kMaxLagrPoints * kMaxLagrPoints; ++i) a.weight[i] = op->weight[i];
     a.herm = op->kind == 3;
+    a.fields = fields;
+    const int64_t between = a.num_elements * a.points;  // of the ping-pong buffers
     const T* cur = in;
     for (int d = 0; d < dim; ++d) {
         a.d = d;
         a.stride = ipow(op->p1, dim - d - 1);
+        a.in_field = d == 0 ? in_field : between;
         if (d == dim - 1) {
+            a.out_field = out_field;
             AMDG_CK(launch_surplus_pass<T, To>(a, cur, out, st));
         } else {
             T* dst = (cur == ta) ? tb : ta;
+            a.out_field = between;
             AMDG_CK(launch_surplus_pass<T, T>(a, cur, dst, st));
             cur = dst;
         }
@@ -697,6 +708,9 @@ amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, c
             o.amp = op->amp;
             if (amdg_status r = run_plan<Tp>(op, m, first, total, np, op->p1, src, 1, nullptr, o, st); r != AMDG_OK)
                 return r;
+            // their surpluses together (the field arrays are `stride` doubles apart, also the FP32 ones)
+            return eval_surplus<double, To>(op, fields + size_t(f_first) * stride, fucoe[f_first], st, f_last - f_first + 1,
+                                            int64_t(stride), int64_t(stride) * int64_t(sizeof(double) / sizeof(To)));
         } else {
             for (int f = f_first; f <= f_last; ++f) {
                 double* acc = static_cast<double*>(op->w_up);
@@ -1072,12 +1086,12 @@ static amdg_status lagr_create(amdg_grid* g, int kind, const double* alpha, doub
         g->ctx->launches++;
         return AMDG_OK;
     };
-    if ((s = upload_both(&op->d_a2p, &op->f_a2p, t.a2p)) != AMDG_OK || (s = upload_both(&op->d_lv, &op->f_lv, t.lv)) != AMDG_OK ||
-        (s = upload_both(&op->d_lvx, &op->f_lvx, t.lvx)) != AMDG_OK ||
-        (s = upload_both(&op->d_lflx, &op->f_lflx, t.lflx)) != AMDG_OK ||
-        (s = upload_both(&op->d_ajump, &op->f_ajump, t.ajump)) != AMDG_OK ||
-        (kind == 1 && ((s = upload_both(&op->d_a2pd, &op->f_a2pd, t.a2pd)) != AMDG_OK ||
-                       (s = upload_both(&op->d_ljv, &op->f_ljv, t.ljv)) != AMDG_OK ||
+    if ((s = upload_both(&op->d_a2p, &op->f_a2p, t.a2p, np * op->p1)) != AMDG_OK || (s = upload_both(&op->d_lv, &op->f_lv, t.lv, np * op->p1)) != AMDG_OK ||
+        (s = upload_both(&op->d_lvx, &op->f_lvx, t.lvx, np * op->p1)) != AMDG_OK ||
+        (s = upload_both(&op->d_lflx, &op->f_lflx, t.lflx, np * op->p1)) != AMDG_OK ||
+        (s = upload_both(&op->d_ajump, &op->f_ajump, t.ajump, np * np)) != AMDG_OK ||
+        (kind == 1 && ((s = upload_both(&op->d_a2pd, &op->f_a2pd, t.a2pd, np * op->p1)) != AMDG_OK ||
+                       (s = upload_both(&op->d_ljv, &op->f_ljv, t.ljv, np * op->p1)) != AMDG_OK ||
                        (s = upload_vec(&op->d_pts, t.pts)) != AMDG_OK || (s = point_sines()) != AMDG_OK)) ||
         (s = upload_df(&op->df_a2p, t.a2p)) != AMDG_OK || (kind == 1 && (s = upload_df(&op->df_a2pd, t.a2pd)) != AMDG_OK) ||
         (s = upload_vec(&op->d_anc_point, t.anc_point)) != AMDG_OK || (s = upload_vec(&op->d_anc_rank, t.anc_rank)) != AMDG_OK ||

@@ -112,9 +112,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1024 / kSweepThreads) sweep_ker
     // the 1D table is blocked by order pair: block (o_s, o_e) holds M[o_s n_from + k][o_e n_to + q]
     // at (k, q), n_from x n_to contiguous
     const int ncols = n_to;
-    const T* mcol = M + size_t(oe) * (n_from * n_to) + qt;
+    const T* mcol = M + size_t(oe) * table_stride<T>(n_from * n_to) + qt;
     const int in_off = outer * n_from * stride + inner;
-    const size_t mstep = size_t(a.n1) * (n_from * n_to);
+    const size_t mstep = size_t(a.n1) * table_stride<T>(n_from * n_to);
     T acc = from_double<T>(0.0);
     // four neighbours per pass: their (element, order) pairs and operands are
     // independent loads issued together; the sum keeps the neighbour order
@@ -227,9 +227,9 @@ __global__ void __launch_bounds__(256) sweep_col_kernel(SweepArgs<T> a) {
     const int beg = lu == 0 ? __ldg(split + et) : __ldg(ptr + et);
     const int end = lu == 2 ? __ldg(split + et) : __ldg(ptr + et + 1);
     const int ncols = NTO;  // blocked 1D table: k-rows of a block are NTO apart
-    const T* mcol = M + size_t(oe) * (n_from * NTO);
+    const T* mcol = M + size_t(oe) * table_stride<T>(n_from * NTO);
     const int in_off = outer * n_from * stride + inner;
-    const size_t mstep = size_t(a.n1) * (n_from * NTO);
+    const size_t mstep = size_t(a.n1) * table_stride<T>(n_from * NTO);
     T acc[NTO];
 #pragma unroll
     for (int q = 0; q < NTO; ++q) acc[q] = from_double<T>(0.0);
@@ -481,6 +481,8 @@ template cudaError_t launch_reduce_rhs<float>(const float*, int, int64_t, int, i
 // kernel (launch_after).
 template <typename Ti, typename To>
 __global__ void __launch_bounds__(256) surplus_pass_kernel(SurplusArgs<Ti> a, const Ti* in, To* out) {
+    in += int64_t(blockIdx.y) * a.in_field;
+    out += int64_t(blockIdx.y) * a.out_field;
     const int64_t gid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t total = a.num_elements * a.points;
     const bool inside = gid < total;
@@ -525,8 +527,9 @@ template <typename Ti, typename To>
 cudaError_t launch_surplus_pass(const SurplusArgs<Ti>& a, const Ti* in, To* out, cudaStream_t st) {
     const int64_t total = a.num_elements * a.points;
     if (total == 0) return cudaSuccess;
-    const int th = ew_threads(total);
-    return launch_after(surplus_pass_kernel<Ti, To>, dim3(unsigned((total + th - 1) / th)), unsigned(th), 0, st, a, in, out);
+    const int th = ew_threads(total * a.fields);
+    return launch_after(surplus_pass_kernel<Ti, To>, dim3(unsigned((total + th - 1) / th), unsigned(a.fields)), unsigned(th), 0,
+                        st, a, in, out);
 }
 
 template cudaError_t launch_surplus_pass<double, double>(const SurplusArgs<double>&, const double*, double*, cudaStream_t);

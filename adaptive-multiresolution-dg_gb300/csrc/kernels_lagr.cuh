@@ -83,6 +83,8 @@ cudaError_t launch_reduce_rhs(const T* buf, int count, int64_t n, int first, int
 template <typename T>
 struct SurplusArgs {
     int dim, d, p1, points, stride;  // p1 points per dimension, points = p1^dim, stride of dimension d
+    int fields;                      // fields passed together, in_field / out_field entries apart
+    int64_t in_field, out_field;
     int64_t num_elements;
     const int32_t* order;
     const int32_t* anc;          // [element][dim][p1]

@@ -50,15 +50,21 @@ struct Fibre {
     const T* in;
     int in_block, stride;
     const T* m;      // block (o_s, o_e) at m + o_s * mstep
-    size_t mstep;
-    double coef;
+    uint32_t mstep;
+    const PlanProduct* product;
     int nf;
 };
 
-// an FP64 multiplication by 1 would still take a slot of the FP64 pipe
+// the product's coefficient where it is not 1 (an FP64 multiplication, or comparison, takes a slot of
+// the FP64 pipe)
 template <typename T>
-__device__ __forceinline__ T times(T v, double c) {
-    return c == 1.0 ? v : scale(v, from_double<T>(c));
+__device__ __forceinline__ T times(T v, const PlanProduct* D) {
+    return D->scaled ? scale(v, from_double<T>(D->coef)) : v;
+}
+
+// x / stride and the remainder, x and stride below 2^16
+__device__ __forceinline__ int quotient(int x, const PlanProduct* D) {
+    return D->stride_inv ? int(__umulhi(uint32_t(x), D->stride_inv)) : x;
 }
 
 template <typename T, int NF, int NT>
@@ -75,17 +81,32 @@ __device__ __forceinline__ Fibre<T> fibre_of(const PlanArgs<T>& a, const PlanPro
     f.in = pen ? a.pen_in : (a.first_sweep ? a.src[D.in] : a.in + int64_t(D.in) * a.in_slice);
     f.in_block = D.in_block;
     f.stride = D.stride;
-    f.m = a.mats[D.mat] + size_t(v.w) * (f.nf * NT);
-    f.mstep = size_t(a.n1) * (f.nf * NT);
-    f.coef = D.coef;
+    const int ts = table_stride<T>((pen ? 3 : NF) * NT);  // the penalty transforms np = 3 entries
+    f.m = a.mats[D.mat] + size_t(v.w) * ts;
+    f.mstep = uint32_t(a.n1) * uint32_t(ts);  // n1 <= 2^16
+    f.product = &D;
     return f;
+}
+
+// A compensated dot product (Ogita, Rump and Oishi's Dot2) of double-float factors: s = (running sum,
+// sum of the errors and of the cross terms); the caller renormalises.  Over the six products of two
+// neighbours its error bound, 36 units of 2^-48, is below that of six double-float multiplications and
+// additions (about 60), for 12 instructions a product instead of 27.
+__device__ __forceinline__ float2 df_product(float2 x, float2 m) {
+    const float p = x.x * m.x;
+    return make_float2(p, fmaf(x.x, m.y, fmaf(x.y, m.x, fmaf(x.x, m.x, -p))));
+}
+__device__ __forceinline__ float2 df_dot(float2 s, float2 x, float2 m) {
+    const float2 p = df_product(x, m);
+    const float2 t = df_two_sum(s.x, p.x);
+    return make_float2(t.x, s.y + (t.y + p.y));
 }
 
 // output entry idx: the neighbours beg + ph, beg + ph + P, ..., four at a time, their operands loaded
 // before the multiply-adds
 template <typename T, int NF, int NT>
 __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, int P) {
-    const int inner = idx % f.stride, rest = idx / f.stride;
+    const int rest = quotient(idx, f.product), inner = idx - rest * f.stride;
     const T* in = f.in + (rest / NT) * NF * f.stride + inner;
     const T* m = f.m + rest % NT;
     T acc;
@@ -100,7 +121,7 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             x[j] = in + int64_t(nb[j].x) * f.in_block;
-            mm[j] = m + size_t(nb[j].y) * f.mstep;
+            mm[j] = m + uint64_t(uint32_t(nb[j].y)) * f.mstep;
         }
         if constexpr (std::is_same<T, float>::value) {
             // FP32: each neighbour's part by itself, then pairwise (fewer roundings on the long sum)
@@ -119,6 +140,23 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
                 for (int k = 1; k < NF; ++k) part[j] = fmaf(xv[j][k], mv[j][k], part[j]);
             }
             acc += (part[0] + part[1]) + (part[2] + part[3]);
+        } else if constexpr (std::is_same<T, float2>::value) {
+            // double-float: two neighbours' products as one compensated dot product, then one addition
+            float2 xv[4][NF], mv[4][NF];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int k = 0; k < NF; ++k) {
+                    xv[j][k] = x[j][k * f.stride];
+                    mv[j][k] = __ldg(mm[j] + k * NT);
+                }
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                float2 s = df_product(xv[j][0], mv[j][0]);
+#pragma unroll
+                for (int k = 1; k < 2 * NF; ++k) s = df_dot(s, xv[j + k / NF][k % NF], mv[j + k / NF][k % NF]);
+                acc = df_add(acc, df_quick_two_sum(s.x, s.y));
+            }
         } else {
             acc = fibre_quad<NF>(x, mm, f.stride, NT, acc);
         }
@@ -126,16 +164,23 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
     for (; i < f.end; i += P) {
         const int2 nb = __ldg(f.nbr + i);
         const T* x = in + int64_t(nb.x) * f.in_block;
-        const T* mm = m + size_t(nb.y) * f.mstep;
+        const T* mm = m + uint64_t(uint32_t(nb.y)) * f.mstep;
         T part;
-        if constexpr (std::is_same<T, float>::value) part = x[0] * __ldg(mm);
-        else part = madd(x[0], __ldg(mm), acc);
+        if constexpr (std::is_same<T, float2>::value) {
+            part = df_product(x[0], __ldg(mm));
 #pragma unroll
-        for (int k = 1; k < NF; ++k) part = madd(x[k * f.stride], __ldg(mm + k * NT), part);
-        if constexpr (std::is_same<T, float>::value) acc += part;
-        else acc = part;
+            for (int k = 1; k < NF; ++k) part = df_dot(part, x[k * f.stride], __ldg(mm + k * NT));
+            acc = df_add(acc, df_quick_two_sum(part.x, part.y));
+        } else {
+            if constexpr (std::is_same<T, float>::value) part = x[0] * __ldg(mm);
+            else part = madd(x[0], __ldg(mm), acc);
+#pragma unroll
+            for (int k = 1; k < NF; ++k) part = madd(x[k * f.stride], __ldg(mm + k * NT), part);
+            if constexpr (std::is_same<T, float>::value) acc += part;
+            else acc = part;
+        }
     }
-    return times(acc, f.coef);
+    return times(acc, f.product);
 }
 template <typename T, int NF, int NT>
 __device__ __forceinline__ T fibre_entry(const Fibre<T>& f, int idx, int ph, int P) {
@@ -163,7 +208,9 @@ __device__ __forceinline__ void add_part(const T (&x)[NF], const T (&m)[NF * NT]
 template <typename T, int NF, int NT>
 __device__ __forceinline__ void fibre_column_n(const Fibre<T>& f, int c, T (&acc)[NT]) {
     constexpr int BS = NF * NT;
-    const T* in = f.in + (c / f.stride) * NF * f.stride + c % f.stride;
+    const int outer = quotient(c, f.product), inner = c - outer * f.stride;
+    const T* in = f.in + outer * NF * f.stride + inner;
+    const bool line = NF == 4 && sizeof(T) == 4 && f.stride == 1;  // a 16-byte line (blocks of a multiple of 4 entries)
 #pragma unroll
     for (int q = 0; q < NT; ++q) set_zero(acc[q]);
     for (int i = f.beg; i < f.end; i += 4) {
@@ -176,13 +223,19 @@ __device__ __forceinline__ void fibre_column_n(const Fibre<T>& f, int c, T (&acc
             const T* x0 = in + int64_t(nb[j].x) * f.in_block;
             const T* x1 = in + int64_t(nb[j + 1].x) * f.in_block;
             T xa[NF], xb[NF], ma[BS], mb[BS];
+            if (line) {
+                const float4 va = *reinterpret_cast<const float4*>(x0), vb = *reinterpret_cast<const float4*>(x1);
+                xa[0] = va.x; xa[1] = va.y; xa[2] = va.z; xa[NF - 1] = va.w;
+                xb[0] = vb.x; xb[1] = vb.y; xb[2] = vb.z; xb[NF - 1] = vb.w;
+            } else {
 #pragma unroll
-            for (int k = 0; k < NF; ++k) {
-                xa[k] = x0[k * f.stride];
-                xb[k] = x1[k * f.stride];
+                for (int k = 0; k < NF; ++k) {
+                    xa[k] = x0[k * f.stride];
+                    xb[k] = x1[k * f.stride];
+                }
             }
-            load_block<T, BS>(f.m + size_t(nb[j].y) * f.mstep, ma);
-            load_block<T, BS>(f.m + size_t(nb[j + 1].y) * f.mstep, mb);
+            load_block<T, BS>(f.m + uint64_t(uint32_t(nb[j].y)) * f.mstep, ma);
+            load_block<T, BS>(f.m + uint64_t(uint32_t(nb[j + 1].y)) * f.mstep, mb);
             T pair[NT];
 #pragma unroll
             for (int q = 0; q < NT; ++q) set_zero(pair[q]);
@@ -193,7 +246,7 @@ __device__ __forceinline__ void fibre_column_n(const Fibre<T>& f, int c, T (&acc
         }
     }
 #pragma unroll
-    for (int q = 0; q < NT; ++q) acc[q] = times(acc[q], f.coef);
+    for (int q = 0; q < NT; ++q) acc[q] = times(acc[q], f.product);
 }
 template <typename T, int NF, int NT>
 __device__ __forceinline__ void fibre_column(const Fibre<T>& f, int c, T (&acc)[NT]) {
@@ -236,7 +289,7 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
     const PlanProduct* prods = a.products + node.first;
     const int64_t r = (int64_t(blockIdx.x) * kSweepCta + threadIdx.x) / P;
     const bool inside = !COL && r < a.num_elements * a.out_block;
-    const int64_t re = inside ? r / a.out_block : 0;
+    const int64_t re = !inside ? 0 : (r < (int64_t(1) << 32) ? int64_t(uint32_t(r) / uint32_t(a.out_block)) : r / a.out_block);
     const bool mine = inside && !long_row(a, node, re);
     Fibre<T> f0{};
     if (mine) f0 = fibre_of<T, NF, NT>(a, prods[0], re);
@@ -289,7 +342,8 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
 #pragma unroll
                 for (int q = 0; q < NT; ++q) sum[q] = add_t(sum[q], part[q]);
                 if (ends) {
-                    const int at = (c / f.stride) * f.stride * NT + c % f.stride;
+                    const int outer = quotient(c, f.product);
+                    const int at = outer * f.stride * NT + c - outer * f.stride;
                     T* o = runs == 1 ? out + e * a.out_block + at : y + g * a.out_block + at;
 #pragma unroll
                     for (int q = 0; q < NT; ++q) o[q * f.stride] = run == 0 ? sum[q] : add_t(o[q * f.stride], sum[q]);
@@ -319,6 +373,16 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
     }
 }
 
+// to_double without conversions, which issue on the FP64 pipe (subnormal parts, not finite ones apart)
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+    const uint32_t b = __float_as_uint(v), e = (b >> 23) & 0xffu;
+    if (e == 0 || e == 0xffu) return (b << 1) ? to_double(v) : __longlong_as_double((long long)(uint64_t(b) << 32));
+    return __longlong_as_double((long long)((uint64_t(b & 0x80000000u) << 32) | (uint64_t(e + (1023 - 127)) << 52) |
+                                            (uint64_t(b & 0x7fffffu) << 29)));
+}
+__device__ __forceinline__ double widen(float2 v) { return widen(v.x) + widen(v.y); }
+
 // What follows the last sweep's sum for output entry (e, idx): parts in product order
 template <typename T>
 __device__ __forceinline__ void plan_epilogue(const PlanArgs<T>& a, const PlanOut& o, int field, int64_t e, int idx,
@@ -335,7 +399,7 @@ __device__ __forceinline__ void plan_epilogue(const PlanArgs<T>& a, const PlanOu
     }
     double* acc = static_cast<double*>(o.acc);
     double v = (o.first || o.mode == kEpiCoef) ? 0.0 : acc[i];
-    for (int p = 0; p < count; ++p) v += to_double(part[p * step]);
+    for (int p = 0; p < count; ++p) v += widen(part[p * step]);
     if (o.mode == kEpiFlux) {
         static_cast<double*>(o.out[field])[i] = v * v * 0.5;  // u^2 / 2
     } else if (o.mode == kEpiCoef) {
@@ -440,7 +504,8 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
             if (!k.live) continue;
             T acc[NT];
             fibre_column<T, NF, NT>(f0, k.item, acc);
-            y += (k.item / f0.stride) * f0.stride * NT + k.item % f0.stride;
+            const int outer = quotient(k.item, f0.product);
+            y += outer * f0.stride * NT + k.item - outer * f0.stride;
 #pragma unroll
             for (int q = 0; q < NT; ++q) y[q * f0.stride] = acc[q];
         } else {
@@ -507,6 +572,8 @@ cudaError_t out_col(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
     const int items = (COL ? a.out_block / NT : W) * P;
     int G = 1;
     while (G < 32 && W == a.out_block && (G + 1) * W <= most && 4 * G * items < 3 * (32 * ((G * items + 31) / 32))) ++G;
+    // ... and CTAs of at least a few warps, while every multiprocessor still gets several
+    while (np * ((G * items + 31) / 32) < 6 && W == a.out_block && 2 * G * W <= most && a.num_elements / (2 * G) >= 1024) G *= 2;
     const int tasks = np * ((G * items + 31) / 32);
     const int rounds = (tasks + kOutCta / 32 - 1) / (kOutCta / 32);
     const int threads = std::max(64, 32 * ((tasks + rounds - 1) / rounds));

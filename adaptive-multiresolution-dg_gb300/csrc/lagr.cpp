@@ -444,6 +444,11 @@ struct PlanBuilder {
 SweepPlan build_sweep_plan(const std::vector<PartialSum>& terms, int first, int count, int dim, int n_in, int n_out,
                            int np, bool node_per_group, std::vector<PlanNode>* nodes,
                            std::vector<PlanProduct>* products) {
+    auto finish = [](PlanProduct* p) {
+        p->stride_inv = p->stride == 1 ? 0u : uint32_t((uint64_t(1) << 32) / uint64_t(p->stride) + 1u);
+        if (p->stride > 1 && (uint64_t(1) << 32) % uint64_t(p->stride) == 0) --p->stride_inv;
+        p->scaled = p->coef != 1.0 ? 1 : 0;
+    };
     PlanBuilder b{terms, dim, n_in, n_out, {}};
     b.products.resize(size_t(dim));
     // the last sweep: per group the products of its terms, in term order
@@ -486,7 +491,8 @@ SweepPlan build_sweep_plan(const std::vector<PartialSum>& terms, int first, int 
     for (int j = 0; j < dim; ++j) {
         plan.offset[j] = int(nodes->size());
         plan.count[j] = int(b.products[size_t(j)].size());
-        for (const auto& list : b.products[size_t(j)]) {
+        for (auto& list : b.products[size_t(j)]) {
+            for (PlanProduct& p : list) finish(&p);
             PlanNode n{int32_t(products->size()), int32_t(list.size()), -1, 0};
             for (const PlanProduct& p : list)
                 if (p.lu != 2) {

@@ -54,6 +54,12 @@ __device__ __forceinline__ double to_double(double v) { return v; }
 __device__ __forceinline__ double to_double(float v) { return double(v); }
 __device__ __forceinline__ double to_double(float2 v) { return double(v.x) + double(v.y); }
 
+// entries between the blocks of a table: FP32 blocks are padded to whole 16-byte loads
+template <typename T>
+__host__ __device__ constexpr int table_stride(int n) {
+    return sizeof(T) == 4 ? (n + 3) / 4 * 4 : n;
+}
+
 // acc + sum over four neighbours j (in order) and k < NF of x[j][k*stride] * m[j][k*ncols],
 // all operands loaded before the first multiply-add.  (The inputs x by plain loads: a kernel launched
 // ahead of its predecessor's end must not read what that one writes through the read-only path.)
@@ -74,11 +80,12 @@ __device__ __forceinline__ T fibre_quad(const T* const* x, const T* const* m, in
     return acc;
 }
 
-// the n entries of a table block (16-byte aligned when n * sizeof(T) is a multiple of 16)
+// the N entries of a table block: 16-byte loads where its stride in the table is a multiple of 16 bytes
 template <typename T, int N>
 __device__ __forceinline__ void load_block(const T* p, T (&v)[N]) {
-    if constexpr ((N * sizeof(T)) % 16 == 0) {
-        constexpr int V = N * sizeof(T) / 16;
+    constexpr int S = table_stride<T>(N);
+    if constexpr ((S * sizeof(T)) % 16 == 0) {
+        constexpr int V = S * sizeof(T) / 16;
         const float4* p4 = reinterpret_cast<const float4*>(p);
         float4 w[V];
 #pragma unroll
@@ -118,8 +125,8 @@ __device__ __forceinline__ void warp_column(const int2* __restrict__ nbr, int fi
             xa[p] = __ldg(x0 + p * stride);
             xb[p] = __ldg(x1 + p * stride);
         }
-        load_block<T, BS>(M + (size_t(n0.y) * mrow + oe) * BS, ma);
-        load_block<T, BS>(M + (size_t(n1.y) * mrow + oe) * BS, mb);
+        load_block<T, BS>(M + (size_t(n0.y) * mrow + oe) * table_stride<T>(BS), ma);
+        load_block<T, BS>(M + (size_t(n1.y) * mrow + oe) * table_stride<T>(BS), mb);
 #pragma unroll
         for (int p = 0; p < NF; ++p)
 #pragma unroll
@@ -135,7 +142,7 @@ __device__ __forceinline__ void warp_column(const int2* __restrict__ nbr, int fi
         T xa[NF], ma[BS];
 #pragma unroll
         for (int p = 0; p < NF; ++p) xa[p] = __ldg(x0 + p * stride);
-        load_block<T, BS>(M + (size_t(n0.y) * mrow + oe) * BS, ma);
+        load_block<T, BS>(M + (size_t(n0.y) * mrow + oe) * table_stride<T>(BS), ma);
 #pragma unroll
         for (int p = 0; p < NF; ++p)
 #pragma unroll
