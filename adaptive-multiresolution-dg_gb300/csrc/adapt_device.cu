@@ -11,10 +11,10 @@
 // rebuilt after every change.  A refinement marks the missing children of the
 // refined leaves into the hash and a list (atomic append), fills holes in one
 // CTA (rounds of "every parent of a new key must exist"), and the new sorted
-// key set is the sort of old and new keys.  A coarsening decides removal by
-// passes over the level sums from the finest down (an element goes when its
-// indicator is below eta, it is not the root, and all its present children
-// went), then compacts by a scan.  Each change synchronises the stream once to
+// key set is the merge of the old keys and the sorted new ones.  A coarsening
+// decides removal by passes over the level sums from the finest down (an
+// element goes when its indicator is below eta, it is not the root, and all its
+// present children went), then compacts by a scan.  Each change synchronises the stream once to
 // learn the new element count; everything else stays on the device.  The
 // results are the host implementation's (csrc/adapt.cpp, csrc/grid.cpp): the
 // same element sets, the same neighbour lists in the same order.
@@ -32,6 +32,7 @@
 #include "kernels.cuh"
 #include "kernels_plan.cuh"
 #include "device_alloc.cuh"
+#include "launch.cuh"
 
 using namespace amdg;
 
@@ -45,6 +46,7 @@ using namespace amdg;
 namespace {
 
 constexpr unsigned long long kEmptyKey = ~0ull;
+constexpr size_t kHashSlot = sizeof(unsigned long long) + sizeof(int32_t);  // a key and its value
 constexpr int kMaxLevels = 17;  // nmax <= 16
 
 cudaStream_t stream_of(const amdg_grid* g) { return static_cast<cudaStream_t>(g->ctx->stream); }
@@ -151,13 +153,15 @@ struct KeyHash {
 
 __device__ __forceinline__ uint64_t hslot(uint64_t k, int bits) { return (k * 0x9E3779B97F4A7C15ull) >> (64 - bits); }
 
-// element index of key k (>= 0), -1 when absent or added by the current refinement
+// element index of key k (>= 0), -1 when absent or added by the current refinement; the value is
+// read beside the key, not after it (a lookup is one trip to the L2 cache instead of two)
 __device__ __forceinline__ int32_t hfind(const KeyHash& h, uint64_t k) {
     uint64_t s = hslot(k, h.bits);
     for (uint64_t i = 0; i <= h.mask; ++i, s = (s + 1) & h.mask) {
         const unsigned long long v = h.key[s];
+        const int32_t w = h.val[s];
         if (v == kEmptyKey) return -1;
-        if (v == k) return h.val[s];
+        if (v == k) return w;
     }
     return -1;
 }
@@ -188,13 +192,6 @@ __global__ void hash_build_kernel(const uint64_t* __restrict__ keys, int64_t E, 
     if (hinsert(h, keys[e], &s)) h.val[s] = int32_t(e);
 }
 
-__global__ void keys_to_order_kernel(const uint64_t* __restrict__ keys, int64_t E, KeyShape ks, int32_t* __restrict__ order) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= E * ks.dim) return;
-    const int64_t e = i / ks.dim;
-    order[i] = ks.field(keys[e], int(i - e * ks.dim));
-}
-
 // ---- indicators ----------------------------------------------------------------
 // sqrt of the block's sum of squares in block order (as element_norm_kernel), plus the second
 // vector's when given, added in that order (DGAdapt::indicator_norm, DGAdapt.cpp:1018-1030)
@@ -216,47 +213,68 @@ __global__ void norms_kernel(const double* __restrict__ u, const double* __restr
     if (!isfinite(v)) st->nonfinite = 1;
 }
 
+// Level statistics of the warp's keys (those with `in`): one atomic per warp and value.  One per
+// element made every element of the set queue at the same few addresses.
+__device__ __forceinline__ void add_level_stats(const KeyShape& ks, uint64_t key, bool in, AdaptStats* st) {
+    if (!__ballot_sync(0xffffffffu, in)) return;
+    const bool first = (threadIdx.x & 31) == 0;
+    int sum = 0;
+    for (int d = 0; d < ks.dim; ++d) {
+        const int l = in ? level_of(ks.field(key, d)) : 0;
+        sum += l;
+        const int s = __reduce_add_sync(0xffffffffu, l), m = __reduce_max_sync(0xffffffffu, l);
+        if (first) {
+            atomicAdd(&st->lev_sum[d], (unsigned long long)s);
+            atomicMax(&st->lev_max[d], m);
+        }
+    }
+    sum = __reduce_max_sync(0xffffffffu, sum);
+    if (first) atomicMax(&st->levsum_max, sum);
+}
+
 // ---- refinement ------------------------------------------------------------------
 // Leaves (fewer present children than possible, DGAdapt::update_leaf) that want refinement get
 // every missing child in every dimension (DGAdapt::refine), appended once to newk.
-__global__ void refine_mark_kernel(const uint64_t* __restrict__ keys, int64_t E, KeyShape ks,
-                                   const double* __restrict__ norms, double eps, const uint8_t* __restrict__ force,
-                                   KeyHash h, uint64_t* __restrict__ newk, AdaptStats* st, int64_t cap,
-                                   uint8_t* __restrict__ refined) {
-    const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const bool want = force ? force[e] != 0 : (norms[e] > eps);
-    refined[e] = 0;
-    if (!want) return;
-    const uint64_t key = keys[e];
-    int existing = 0, total = 0, ch[2];
-    for (int d = 0; d < ks.dim; ++d) {
-        const int nc = children_of(ks.field(key, d), ks.nmax, ch);
-        total += nc;
-        for (int c = 0; c < nc; ++c) existing += hfind(h, ks.with(key, d, ch[c])) >= 0 ? 1 : 0;
-    }
-    if (existing >= total) return;
-    refined[e] = 1;
-    for (int d = 0; d < ks.dim; ++d) {
-        const int nc = children_of(ks.field(key, d), ks.nmax, ch);
-        for (int c = 0; c < nc; ++c) {
-            const uint64_t ck = ks.with(key, d, ch[c]);
-            if (hfind(h, ck) >= 0) continue;
-            uint64_t slot;
-            if (!hinsert(h, ck, &slot)) continue;
-            const long long i = (long long)atomicAdd(&st->count, 1ull);
-            if (i < cap) newk[i] = ck;
-            else atomicOr(&st->err, 1);
+// `width` lanes (a power of two, 2 dim or more) share an element, one child each: the lookups of an
+// element are one trip to memory, not 2 dim in a row.
+__global__ void refine_mark_kernel(const uint64_t* keys, int64_t E, KeyShape ks, const double* norms, double eps,
+                                   const uint8_t* force, KeyHash h, uint64_t* newk, AdaptStats* st, int64_t cap,
+                                   uint8_t* refined, int width) {
+    const int64_t gid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, j = lane & (width - 1);
+    const int64_t e = gid / width;
+    wait_for_previous();
+    const bool want = e < E && (force ? force[e] != 0 : (norms[e] > eps));
+    uint64_t ck = 0;
+    bool child = false, there = false;
+    if (want && j < 2 * ks.dim) {
+        const uint64_t key = keys[e];
+        int ch[2];
+        const int d = j >> 1, nc = children_of(ks.field(key, d), ks.nmax, ch);
+        child = (j & 1) < nc;
+        if (child) {
+            ck = ks.with(key, d, ch[j & 1]);
+            there = hfind(h, ck) >= 0;
         }
+    }
+    const unsigned group = (width == 32 ? 0xffffffffu : ((1u << width) - 1u)) << (lane - j);
+    const bool leaf = (__ballot_sync(0xffffffffu, child && !there) & group) != 0;
+    if (e < E && j == 0) refined[e] = leaf ? 1 : 0;
+    uint64_t slot;
+    if (child && !there && hinsert(h, ck, &slot)) {
+        const long long i = (long long)atomicAdd(&st->count, 1ull);
+        if (i < cap) newk[i] = ck;
+        else atomicOr(&st->err, 1);
     }
 }
 
 // Hole filling (DGAdapt::check_hole) in one CTA: every parent of a new key must be present;
 // rounds over the keys the previous round added, until a round adds none.  Then the level
 // statistics of the added keys.
-__global__ void __launch_bounds__(1024) hole_fill_kernel(KeyShape ks, KeyHash h, uint64_t* __restrict__ newk,
-                                                         AdaptStats* st, int64_t cap) {
+__global__ void __launch_bounds__(1024) hole_fill_kernel(KeyShape ks, KeyHash h, uint64_t* newk, AdaptStats* st,
+                                                         int64_t cap) {
     __shared__ long long s_hi;
+    wait_for_previous();
     long long lo = 0;
     int round = 0;
     for (;; ++round) {
@@ -287,34 +305,33 @@ __global__ void __launch_bounds__(1024) hole_fill_kernel(KeyShape ks, KeyHash h,
     }
     __syncthreads();
     const long long n = s_hi < cap ? s_hi : cap;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint64_t key = newk[i];
-        int sum = 0;
-        for (int d = 0; d < ks.dim; ++d) {
-            const int l = level_of(ks.field(key, d));
-            sum += l;
-            atomicAdd(&st->lev_sum[d], (unsigned long long)l);
-            atomicMax(&st->lev_max[d], l);
-        }
-        atomicMax(&st->levsum_max, sum);
+    for (long long i0 = 0; i0 < n; i0 += blockDim.x) {  // whole warps: the sums are taken per warp
+        const long long i = i0 + threadIdx.x;
+        add_level_stats(ks, i < n ? newk[i] : 0, i < n, st);
     }
 }
 
-__global__ void concat_keys_kernel(const uint64_t* __restrict__ a, int64_t na, const uint64_t* __restrict__ b, int64_t nb,
-                                   uint64_t* __restrict__ out) {
+// The new element set: old and added keys, both sorted and without common keys, merged by rank (a
+// key's place is its own index plus the number of the other list's keys below it).  Writes the
+// keys, their 1D orders and the old element of each (-1: added).
+__global__ void merge_keys_kernel(const uint64_t* old, int64_t E, const uint64_t* added, int64_t n, KeyShape ks,
+                                  uint64_t* out, int32_t* map, int32_t* order) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < na) out[i] = a[i];
-    else if (i < na + nb) out[i] = b[i - na];
-}
-
-// new element -> old element (-1: added) through the old set's hash, and the new orders
-__global__ void map_from_hash_kernel(const uint64_t* __restrict__ keys, int64_t E, KeyShape ks, KeyHash h,
-                                     int32_t* __restrict__ map, int32_t* __restrict__ order) {
-    const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const uint64_t key = keys[e];
-    map[e] = hfind(h, key);
-    for (int d = 0; d < ks.dim; ++d) order[e * ks.dim + d] = ks.field(key, d);
+    wait_for_previous();
+    if (i >= E + n) return;
+    const bool is_old = i < E;
+    const uint64_t key = is_old ? old[i] : added[i - E];
+    const uint64_t* other = is_old ? added : old;
+    int64_t lo = 0, hi = is_old ? n : E;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (other[mid] < key) lo = mid + 1;
+        else hi = mid;
+    }
+    const int64_t r = lo + (is_old ? i : i - E);
+    out[r] = key;
+    map[r] = is_old ? int32_t(i) : -1;
+    for (int d = 0; d < ks.dim; ++d) order[r * ks.dim + d] = ks.field(key, d);
 }
 
 // ---- coarsening ------------------------------------------------------------------
@@ -359,16 +376,10 @@ __global__ void coarsen_stats_kernel(const uint64_t* __restrict__ keys, int64_t 
                                      uint64_t* __restrict__ missed, int64_t missed_cap, AdaptStats* st) {
     const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (e == 0) st->count = pos[E];
-    if (e >= E || removed[e]) return;
-    const uint64_t key = keys[e];
-    int sum = 0;
-    for (int d = 0; d < ks.dim; ++d) {
-        const int l = level_of(ks.field(key, d));
-        sum += l;
-        atomicAdd(&st->lev_sum[d], (unsigned long long)l);
-        atomicMax(&st->lev_max[d], l);
-    }
-    atomicMax(&st->levsum_max, sum);
+    const bool kept = e < E && !removed[e];
+    const uint64_t key = kept ? keys[e] : 0;
+    add_level_stats(ks, key, kept, st);
+    if (!kept) return;
     if (missed_eps > 0.0 && norms[e] > missed_eps) {
         int existing = 0, total = 0, ch[2];
         for (int d = 0; d < ks.dim; ++d) {
@@ -386,82 +397,115 @@ __global__ void coarsen_stats_kernel(const uint64_t* __restrict__ keys, int64_t 
     }
 }
 
-// The whole coarsening of a small element set in one CTA: the level-sum passes (finest first,
-// separated by barriers), the keep flags and their exclusive scan (a block scan over
-// kSmallCoarsenItems elements per thread), and the statistics of the kept set -- the same flags,
-// positions and statistics as coarsen_pass_kernel + keep_flags_kernel + the device scan +
-// coarsen_stats_kernel, without their launches.
+// The whole coarsening of a small element set in one CTA: the same flags, positions and statistics
+// as coarsen_pass_kernel + keep_flags_kernel + the device scan + coarsen_stats_kernel, without their
+// launches.  "Some child is kept" is pushed up by the kept elements, not looked up by their parents:
+// an element that the indicator keeps marks its parents (a byte of shared memory each) before the
+// first pass, so a pass over a level sum only reads the marks of its candidates, and only a
+// candidate that stays has lookups left to do.  With every element's key read and every candidate's
+// children looked up in each pass, and one atomic per element and statistic, the kernel took
+// 23 us at 1,168 elements and 86 us at 3,880; it takes 14 and 24 us.
 constexpr int kSmallCoarsenThreads = 1024, kSmallCoarsenItems = 8;
 constexpr int64_t kSmallCoarsenMax = int64_t(kSmallCoarsenThreads) * kSmallCoarsenItems;
-__global__ void __launch_bounds__(kSmallCoarsenThreads)
-    coarsen_small_kernel(const uint64_t* __restrict__ keys, int64_t E, KeyShape ks, const double* __restrict__ norms,
-                         double eta, int levsum_max, KeyHash h, uint8_t* __restrict__ removed,
-                         int32_t* __restrict__ pos, double missed_eps, uint64_t* __restrict__ missed,
+
+// inclusive scan over the lanes of a warp
+template <class T>
+__device__ __forceinline__ T warp_scan(T v) {
+#pragma unroll
+    for (int q = 1; q < 32; q <<= 1) {
+        const T u = __shfl_up_sync(0xffffffffu, v, q);
+        if (int(threadIdx.x & 31) >= q) v += u;
+    }
+    return v;
+}
+
+// sum of `mine` over the warps below this one (32 warps, one value each) and over all of them
+template <class T>
+__device__ __forceinline__ T warps_before(T mine, T* totals, T* all) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) totals[warp] = mine;
+    __syncthreads();
+    const T t = totals[lane], upto = warp_scan(t);
+    *all = __shfl_sync(0xffffffffu, upto, 31);
+    return __shfl_sync(0xffffffffu, upto - t, warp);
+}
+
+__global__ void __launch_bounds__(kSmallCoarsenThreads, 1)
+    coarsen_small_kernel(const uint64_t* keys, int64_t E, KeyShape ks, const double* norms, double eta, int levsum_max,
+                         KeyHash h, uint8_t* removed, int32_t* pos, double missed_eps, uint64_t* missed,
                          int64_t missed_cap, AdaptStats* st) {
+    __shared__ uint8_t held[kSmallCoarsenMax];  // some child of the element is kept
+    __shared__ uint8_t gone[kSmallCoarsenMax];  // the element is removed
     const int tid = threadIdx.x;
-    for (int64_t e = tid; e < E; e += kSmallCoarsenThreads) removed[e] = 0;
+    wait_for_previous();
+    for (int e = tid; e < int(E); e += kSmallCoarsenThreads) held[e] = gone[e] = 0;
+    __syncthreads();
+    auto mark_parents = [&](uint64_t key) {
+        for (int d = 0; d < ks.dim; ++d) {
+            const int o = ks.field(key, d);
+            if (o == 0) continue;
+            const int32_t p = hfind(h, ks.with(key, d, parent_of(o)));
+            if (p >= 0) held[p] = 1;
+        }
+    };
+    int level[kSmallCoarsenItems];  // level sum of a candidate, 0: no candidate
+#pragma unroll
+    for (int i = 0; i < kSmallCoarsenItems; ++i) {
+        const int e = tid + i * kSmallCoarsenThreads;
+        level[i] = 0;
+        if (e >= int(E)) continue;
+        const uint64_t key = keys[e];
+        if (norms[e] < eta)
+            for (int d = 0; d < ks.dim; ++d) level[i] += level_of(ks.field(key, d));
+        if (level[i] == 0) mark_parents(key);
+    }
     __syncthreads();
     for (int L = levsum_max; L >= 1; --L) {
-        for (int64_t e = tid; e < E; e += kSmallCoarsenThreads) {
-            const uint64_t key = keys[e];
-            int sum = 0, mx = 0;
-            for (int d = 0; d < ks.dim; ++d) {
-                const int l = level_of(ks.field(key, d));
-                sum += l;
-                mx = l > mx ? l : mx;
-            }
-            if (sum != L || mx == 0 || !(norms[e] < eta)) continue;
-            bool keep_it = false;
-            int ch[2];
-            for (int d = 0; d < ks.dim && !keep_it; ++d) {
-                const int nc = children_of(ks.field(key, d), ks.nmax, ch);
-                for (int c = 0; c < nc; ++c) {
-                    const int32_t i = hfind(h, ks.with(key, d, ch[c]));
-                    if (i >= 0 && !removed[i]) keep_it = true;
-                }
-            }
-            if (!keep_it) removed[e] = 1;
+#pragma unroll
+        for (int i = 0; i < kSmallCoarsenItems; ++i) {
+            if (level[i] != L) continue;
+            const int e = tid + i * kSmallCoarsenThreads;
+            if (held[e]) mark_parents(keys[e]);
+            else gone[e] = 1;
         }
-        __syncthreads();  // pass L - 1 reads the flags of pass L
+        __syncthreads();  // pass L - 1 reads the marks of pass L
     }
-    using Scan = cub::BlockScan<int, kSmallCoarsenThreads>;
-    __shared__ typename Scan::TempStorage scan_tmp;
-    int v[kSmallCoarsenItems];
+    // kept positions: a warp's kSmallCoarsenItems x 32 elements by ballots, then the warps' totals
+    __shared__ int totals[32];
+    const int lane = tid & 31, warp = tid >> 5, first = warp * 32 * kSmallCoarsenItems + lane;
+    int v[kSmallCoarsenItems], mine = 0;
 #pragma unroll
     for (int i = 0; i < kSmallCoarsenItems; ++i) {
-        const int64_t e = int64_t(tid) * kSmallCoarsenItems + i;
-        v[i] = (e < E && !removed[e]) ? 1 : 0;
+        const int e = first + 32 * i;
+        const unsigned kept = __ballot_sync(0xffffffffu, e < int(E) && !gone[e]);
+        v[i] = mine + __popc(kept & ((1u << lane) - 1u));
+        mine += __popc(kept);
     }
-    int total = 0;
-    Scan(scan_tmp).ExclusiveSum(v, v, total);
+    int total;
+    const int base = warps_before(mine, totals, &total);
 #pragma unroll
     for (int i = 0; i < kSmallCoarsenItems; ++i) {
-        const int64_t e = int64_t(tid) * kSmallCoarsenItems + i;
-        if (e < E) pos[e] = v[i];
+        const int e = first + 32 * i;
+        if (e < int(E)) pos[e] = base + v[i];
     }
     if (tid == 0) {
         pos[E] = total;
         st->count = (unsigned long long)total;
     }
-    for (int64_t e = tid; e < E; e += kSmallCoarsenThreads) {
-        if (removed[e]) continue;
-        const uint64_t key = keys[e];
-        int sum = 0;
-        for (int d = 0; d < ks.dim; ++d) {
-            const int l = level_of(ks.field(key, d));
-            sum += l;
-            atomicAdd(&st->lev_sum[d], (unsigned long long)l);
-            atomicMax(&st->lev_max[d], l);
-        }
-        atomicMax(&st->levsum_max, sum);
-        if (missed_eps > 0.0 && norms[e] > missed_eps) {
+    for (int e0 = 0; e0 < int(E); e0 += kSmallCoarsenThreads) {
+        const int e = e0 + tid;
+        const bool kept = e < int(E) && !gone[e];
+        const uint64_t key = kept ? keys[e] : 0;
+        add_level_stats(ks, key, kept, st);
+        if (e < int(E)) removed[e] = kept ? 0 : 1;
+        if (kept && missed_eps > 0.0 && norms[e] > missed_eps) {
             int existing = 0, tot = 0, ch[2];
             for (int d = 0; d < ks.dim; ++d) {
                 const int nc = children_of(ks.field(key, d), ks.nmax, ch);
                 tot += nc;
                 for (int c = 0; c < nc; ++c) {
                     const int32_t i = hfind(h, ks.with(key, d, ch[c]));
-                    existing += (i >= 0 && !removed[i]) ? 1 : 0;
+                    existing += (i >= 0 && !gone[i]) ? 1 : 0;
                 }
             }
             if (existing < tot) {
@@ -512,13 +556,14 @@ __device__ __forceinline__ LevelRange level_range(int l, int nmax, int64_t a0, i
     LevelRange r;
     const int64_t one = int64_t(1) << nmax;
     r.cnt = 1 << (l - 1);
-    const int64_t w = one >> (l - 1);
-    r.first = int(a0 / w);
-    r.last = int((b0 - 1) / w);
+    const int sh = nmax - l + 1;  // intervals of 2^sh units
+    const int64_t in = (int64_t(1) << sh) - 1;
+    r.first = int(a0 >> sh);
+    r.last = int((b0 - 1) >> sh);
     r.lo = r.first;
     r.hi = r.last;
-    if (a0 % w == 0 && r.first >= 1) --r.lo;
-    if (b0 % w == 0 && r.last + 1 < r.cnt) ++r.hi;
+    if ((a0 & in) == 0 && r.first >= 1) --r.lo;
+    if ((b0 & in) == 0 && r.last + 1 < r.cnt) ++r.hi;
     r.wrap_lo = b0 == one && r.lo > 0;
     r.wrap_hi = a0 == 0 && r.hi < r.cnt - 1;
     return r;
@@ -570,10 +615,12 @@ __device__ __forceinline__ int cand_order(const LevelCands& c, int i) {
     return c.base + c.lo + (i - c.wl);
 }
 
-// One warp per row (element, dimension): every level's candidates looked up 32 at a time, the
-// present ones counted (fill == nullptr) or written in order (ballot prefix) -- no per-thread
-// chains of dependent lookups.  Returns, on lane 0, the vol / flx counts and the counts at levels
-// up to the element's own (the split between the "U" and "L" parts).
+// One warp per row (element, dimension): the candidates of all levels in one sequence, looked up 32 at a
+// time, the present ones counted (out == nullptr) or written in order (ballot prefix).  Returns the
+// vol / flx counts and the counts at levels up to the element's own (the split between the "U" and
+// "L" parts).  Most rows have a few candidates on each level: taken level by level, a row waited
+// for nmax + 1 lookups one after the other (the fill 32 us at 3,880 elements in two dimensions, cold
+// caches, 14 us at 390; 22 and 10 us with the levels in one sequence).
 struct RowOut {
     int2* vol;
     int2* flx;
@@ -588,36 +635,46 @@ __device__ __forceinline__ void row_lists(const TopoArgs& A, int64_t e, int t, c
     int64_t a0, b0;
     support_of(oi, nmax, &a0, &b0);
     int nv = 0, nf = 0, sv = 0, sf = 0;
-    for (int l = 0; l <= nmax; ++l) {
-        const LevelCands c = level_cands(l, nmax, a0, b0);
-        for (int base = 0; base < c.n; base += 32) {
-            const int i = base + lane;
-            int s = -1, o = 0;
-            if (i < c.n) {
-                o = cand_order(c, i);
-                s = hfind(A.h, A.ks.with(key, t, o));
+    // lane l holds the number of candidates up to level l; those of the "U" part come first
+    const int upto = warp_scan(lane <= nmax ? level_cands(lane, nmax, a0, b0).n : 0);
+    const int total = __shfl_sync(0xffffffffu, upto, nmax), upper = __shfl_sync(0xffffffffu, upto, own);
+    for (int base = 0; base < total; base += 32) {
+        const int i = base + lane;
+        int l = 0, before = 0;  // level of candidate i, candidates of the levels below
+        for (int q = 0; q < nmax; ++q) {
+            const int u = __shfl_sync(0xffffffffu, upto, q);
+            if (u <= i) {
+                l = q + 1;
+                before = u;
             }
-            const bool inv = s >= 0 && o >= c.vfirst && o <= c.vlast;
-            const unsigned bf = __ballot_sync(0xffffffffu, s >= 0);
-            const unsigned bv = __ballot_sync(0xffffffffu, inv);
-            if (out) {
-                const unsigned below = (1u << lane) - 1u;
-                if (s >= 0) {
-                    const int pf = nf + __popc(bf & below);
-                    if (pf < out->fmax) out->flx[pf] = make_int2(s, o);
-                }
-                if (inv) {
-                    const int pv = nv + __popc(bv & below);
-                    if (pv < out->vmax) out->vol[pv] = make_int2(s, o);
-                }
+        }
+        int s = -1, o = 0;
+        bool inv = false;
+        if (i < total) {
+            const LevelCands c = level_cands(l, nmax, a0, b0);
+            o = cand_order(c, i - before);
+            s = hfind(A.h, A.ks.with(key, t, o));
+            inv = s >= 0 && o >= c.vfirst && o <= c.vlast;
+        }
+        const unsigned bf = __ballot_sync(0xffffffffu, s >= 0);
+        const unsigned bv = __ballot_sync(0xffffffffu, inv);
+        if (out) {
+            const unsigned below = (1u << lane) - 1u;
+            if (s >= 0) {
+                const int pf = nf + __popc(bf & below);
+                if (pf < out->fmax) out->flx[pf] = make_int2(s, o);
             }
-            nf += __popc(bf);
-            nv += __popc(bv);
+            if (inv) {
+                const int pv = nv + __popc(bv & below);
+                if (pv < out->vmax) out->vol[pv] = make_int2(s, o);
+            }
         }
-        if (l <= own) {
-            sv = nv;
-            sf = nf;
-        }
+        nf += __popc(bf);
+        nv += __popc(bv);
+        const int left = upper - base;
+        const unsigned um = left >= 32 ? 0xffffffffu : left > 0 ? (1u << left) - 1u : 0u;
+        sf += __popc(bf & um);
+        sv += __popc(bv & um);
     }
     *nv_out = nv;
     *nf_out = nf;
@@ -625,10 +682,10 @@ __device__ __forceinline__ void row_lists(const TopoArgs& A, int64_t e, int t, c
     *sf_out = sf;
 }
 
-__global__ void topo_count_kernel(TopoArgs A, int32_t* __restrict__ vcnt, int32_t* __restrict__ fcnt,
-                                  int32_t* __restrict__ long_count) {
+__global__ void topo_count_kernel(TopoArgs A, int32_t* vcnt, int32_t* fcnt, int32_t* long_count) {
     const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int dim = A.ks.dim;
+    wait_for_previous();
     if (row > A.E * dim) return;  // whole warps: the row test is uniform
     if (row == A.E * dim) {
         if ((threadIdx.x & 31) == 0) vcnt[row] = fcnt[row] = 0;
@@ -644,13 +701,14 @@ __global__ void topo_count_kernel(TopoArgs A, int32_t* __restrict__ vcnt, int32_
     }
 }
 
-__global__ void topo_fill_kernel(TopoArgs A, const int32_t* __restrict__ vol_ptr, const int32_t* __restrict__ flx_ptr,
-                                 int2* __restrict__ vol_nbr, int2* __restrict__ flx_nbr, int32_t* __restrict__ vol_split,
-                                 int32_t* __restrict__ flx_split, int64_t vol_cap, int64_t flx_cap, int* err,
-                                 RowRec* __restrict__ rows, int32_t* long_count, int32_t* long_rows,
+__global__ void topo_fill_kernel(TopoArgs A, const int32_t* vol_ptr, const int32_t* flx_ptr,
+                                 int2* vol_nbr, int2* flx_nbr, int32_t* vol_split,
+                                 int32_t* flx_split, int64_t vol_cap, int64_t flx_cap, int* err,
+                                 RowRec* rows, int32_t* long_count, int32_t* long_rows,
                                  int64_t long_stride) {
     const int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int dim = A.ks.dim;
+    wait_for_previous();
     if (row >= A.E * dim) return;
     const int64_t v0 = vol_ptr[row], f0 = flx_ptr[row];
     const int64_t v1 = vol_ptr[row + 1], f1 = flx_ptr[row + 1];
@@ -677,22 +735,21 @@ __global__ void topo_fill_kernel(TopoArgs A, const int32_t* __restrict__ vol_ptr
 
 // surplus ancestors anc[e][d][ic]: the element owning surplus point ic of e along d
 // (LagrInterpolation::eval_fp_to_coe_D_Lag, Interplation.cpp:1318-1376); -1 for level 0
-__global__ void ancestors_kernel(TopoArgs A, const int32_t* __restrict__ anc_order, int p1, int32_t* __restrict__ anc,
-                                 int* err) {
+__global__ void ancestors_kernel(TopoArgs A, const int32_t* anc_order, int p1, int32_t* anc, int* err) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int dim = A.ks.dim;
-    if (i >= A.E * dim) return;
-    const int64_t e = i / dim;
-    const int d = int(i - e * dim);
+    wait_for_previous();
+    if (i >= A.E * dim * p1) return;
+    const int64_t row = i / p1, e = row / dim;
+    const int ic = int(i - row * p1), d = int(row - e * dim);
     const uint64_t key = A.keys[e];
     const int o = A.ks.field(key, d);
-    int32_t* out = anc + i * p1;
-    for (int ic = 0; ic < p1; ++ic) {
-        if (o == 0) { out[ic] = -1; continue; }
-        const int32_t s = hfind(A.h, A.ks.with(key, d, anc_order[o * p1 + ic]));
+    int32_t s = -1;
+    if (o != 0) {
+        s = hfind(A.h, A.ks.with(key, d, anc_order[o * p1 + ic]));
         if (s < 0) atomicOr(err, 2);
-        out[ic] = s;
     }
+    anc[i] = s;
 }
 
 __global__ void parent_table_kernel(TopoArgs A, int32_t* __restrict__ pg) {
@@ -867,22 +924,21 @@ amdg_status grid_hash(amdg_grid* g) {
     const int64_t need = 2 * (1 + 2 * int64_t(g->host.dim)) * std::max<int64_t>(E, 1);
     if (need > d.hcap) {
         cudaFree(d.hkey);
-        cudaFree(d.hval);
         d.hkey = nullptr;
         d.hval = nullptr;
         d.hcap = 0;
         int bits = 6;
         while ((int64_t(1) << bits) < need + need / 2) ++bits;
         const int64_t cap = int64_t(1) << bits;
-        if (amdg::device_malloc(&d.hkey, size_t(cap) * sizeof(unsigned long long)) != cudaSuccess ||
-            amdg::device_malloc(&d.hval, size_t(cap) * sizeof(int32_t)) != cudaSuccess)
+        // the values lie behind the keys: one fill empties both
+        if (amdg::device_malloc(reinterpret_cast<void**>(&d.hkey), size_t(cap) * kHashSlot) != cudaSuccess)
             return fail(AMDG_ERR_NOMEM, "cudaMalloc failed (element hash)");
+        d.hval = reinterpret_cast<int32_t*>(d.hkey + cap);
         d.hcap = cap;
         d.hbits = bits;
     }
     cudaStream_t st = stream_of(g);
-    AMDG_CK(cudaMemsetAsync(d.hkey, 0xFF, size_t(d.hcap) * sizeof(unsigned long long), st));
-    AMDG_CK(cudaMemsetAsync(d.hval, 0xFF, size_t(d.hcap) * sizeof(int32_t), st));
+    AMDG_CK(cudaMemsetAsync(d.hkey, 0xFF, size_t(d.hcap) * kHashSlot, st));
     if (E > 0) {
         hash_build_kernel<<<blocks_for(E, 256), 256, 0, st>>>(d.key, E, hash_of(g));
         AMDG_CK(cudaGetLastError());
@@ -1006,11 +1062,12 @@ amdg_status grid_device_refine(amdg_grid* g, double eps, const uint8_t* d_force,
     AdaptStats* dst = static_cast<AdaptStats*>(d.stats);
     AMDG_CK(cudaMemsetAsync(dst, 0, kStatsReset, st));
     if (E > 0) {
-        refine_mark_kernel<<<blocks_for(E, 128), 128, 0, st>>>(d.key, E, ks, d_force ? nullptr : g->d_norms, eps,
-                                                               d_force, hash_of(g), d.newk, dst, d.new_cap, d.flag);
-        AMDG_CK(cudaGetLastError());
-        hole_fill_kernel<<<1, 1024, 0, st>>>(ks, hash_of(g), d.newk, dst, d.new_cap);
-        AMDG_CK(cudaGetLastError());
+        int width = 2;  // lanes per element: 12 -> 6 us at 2,104 elements in three dimensions
+        while (width < 2 * ks.dim) width *= 2;
+        AMDG_CK(launch_after(refine_mark_kernel, dim3(blocks_for(E * width, 128)), 128, 0, st, d.key, E, ks,
+                             d_force ? nullptr : g->d_norms, eps, d_force, hash_of(g), d.newk, dst, d.new_cap, d.flag,
+                             width));
+        AMDG_CK(launch_after(hole_fill_kernel, dim3(1), 1024, 0, st, ks, hash_of(g), d.newk, dst, d.new_cap));
         g->ctx->launches += 2;
     }
     AdaptStats hs;
@@ -1030,19 +1087,18 @@ amdg_status grid_device_refine(amdg_grid* g, double eps, const uint8_t* d_force,
     if ((s = ensure_keys(g, En, true)) != AMDG_OK || (s = ensure_set_arrays(g, En)) != AMDG_OK ||
         (s = grid_reserve_remap(g, En)) != AMDG_OK)
         return s;
-    size_t temp = 0;
-    AMDG_CK(cub::DeviceRadixSort::SortKeys(nullptr, temp, d.key_alt, d.key, int(En), 0, ks.dim * ks.nmax, st));
-    if ((s = grow_temp(d, temp)) != AMDG_OK) return s;
-    // old and new keys side by side in key_alt, then sorted into key (keys use dim * nmax bits);
-    // the old keys are not needed again: the map comes from the old set's hash
-    concat_keys_kernel<<<blocks_for(En, 256), 256, 0, st>>>(d.key, E, d.newk, n_new, d.key_alt);
-    AMDG_CK(cudaGetLastError());
+    // only the added keys are sorted (keys use dim * nmax bits), into the scratch behind the sort's own
     const int bits = ks.dim * ks.nmax;
-    size_t tb = d.temp_bytes;
-    AMDG_CK(cub::DeviceRadixSort::SortKeys(d.temp, tb, d.key_alt, d.key, int(En), 0, bits, st));
-    map_from_hash_kernel<<<blocks_for(En, 256), 256, 0, st>>>(d.key, En, ks, hash_of(g), g->d_map, g->d_order);
-    AMDG_CK(cudaGetLastError());
-    g->ctx->launches += 3;
+    const size_t list = (size_t(n_new) * sizeof(uint64_t) + 255) / 256 * 256;
+    size_t temp = 0;
+    AMDG_CK(cub::DeviceRadixSort::SortKeys(nullptr, temp, d.newk, d.newk, int(n_new), 0, bits, st));
+    if ((s = grow_temp(d, list + temp)) != AMDG_OK) return s;
+    uint64_t* sorted = static_cast<uint64_t*>(d.temp);
+    AMDG_CK(cub::DeviceRadixSort::SortKeys(static_cast<char*>(d.temp) + list, temp, d.newk, sorted, int(n_new), 0, bits, st));
+    AMDG_CK(launch_after(merge_keys_kernel, dim3(blocks_for(En, 128)), 128, 0, st, d.key, E, sorted, n_new, ks, d.key_alt,
+                         g->d_map, g->d_order));
+    g->ctx->launches += 2;
+    std::swap(d.key, d.key_alt);
     if ((s = grid_apply_remap(g, En)) != AMDG_OK) return s;
     for (int k = 0; k < ks.dim; ++k) {
         g->lev_sum[k] += hs.lev_sum[k];
@@ -1069,10 +1125,8 @@ amdg_status grid_device_coarsen(amdg_grid* g, double eta, double missed_eps, int
         return AMDG_OK;
     }
     if (E <= kSmallCoarsenMax) {  // one CTA does it all
-        coarsen_small_kernel<<<1, kSmallCoarsenThreads, 0, st>>>(d.key, E, ks, g->d_norms, eta, g->levsum_max,
-                                                                  hash_of(g), d.flag, d.pos, missed_eps, d.missed,
-                                                                  d.missed_cap, dst);
-        AMDG_CK(cudaGetLastError());
+        AMDG_CK(launch_after(coarsen_small_kernel, dim3(1), kSmallCoarsenThreads, 0, st, d.key, E, ks, g->d_norms, eta,
+                             g->levsum_max, hash_of(g), d.flag, d.pos, missed_eps, d.missed, d.missed_cap, dst));
         g->ctx->launches++;
     } else {
         AMDG_CK(cudaMemsetAsync(d.flag, 0, size_t(E), st));
@@ -1165,29 +1219,38 @@ void transform_topology_bounds(const amdg_grid* g, int64_t* vol_pairs, int64_t* 
 }
 
 // Exclusive scans of the vol and flx row counts (n entries each) in one CTA, for small element
-// sets: the results of the two device-wide scans without their launches.
-__global__ void __launch_bounds__(kSmallCoarsenThreads)
-    scan_pair_small_kernel(const int32_t* __restrict__ a, const int32_t* __restrict__ b, int64_t n,
-                           int32_t* __restrict__ sa, int32_t* __restrict__ sb) {
-    using Scan = cub::BlockScan<int, kSmallCoarsenThreads>;
-    __shared__ typename Scan::TempStorage tmp;
-    const int tid = threadIdx.x;
-    for (int which = 0; which < 2; ++which) {
-        const int32_t* in = which ? b : a;
-        int32_t* out = which ? sb : sa;
-        int v[kSmallCoarsenItems];
+// sets: the results of the two device-wide scans without their launches.  Both counts of a row in
+// one 64-bit sum (the lists hold fewer than 2^31 entries each); a warp scans consecutive rows, 32
+// side by side, so that its loads and stores are whole lines (eight consecutive rows per thread and
+// one scan per array: 11 us at 7,761 rows, cold caches; 8 us this way).
+__global__ void __launch_bounds__(kSmallCoarsenThreads, 1)
+    scan_pair_small_kernel(const int32_t* a, const int32_t* b, int64_t n, int32_t* sa, int32_t* sb) {
+    __shared__ unsigned long long totals[32];
+    const int items = int((n + kSmallCoarsenThreads - 1) / kSmallCoarsenThreads);  // rows per thread
+    const int first = (threadIdx.x >> 5) * 32 * items + (threadIdx.x & 31);
+    unsigned long long v[kSmallCoarsenItems], mine = 0;
+    wait_for_previous();
 #pragma unroll
-        for (int i = 0; i < kSmallCoarsenItems; ++i) {
-            const int64_t r = int64_t(tid) * kSmallCoarsenItems + i;
-            v[i] = r < n ? in[r] : 0;
-        }
-        Scan(tmp).ExclusiveSum(v, v);
+    for (int i = 0; i < kSmallCoarsenItems; ++i) {
+        const int r = first + 32 * i;
+        v[i] = i < items && r < int(n) ? (unsigned long long)(unsigned(b[r])) << 32 | unsigned(a[r]) : 0ull;
+    }
 #pragma unroll
-        for (int i = 0; i < kSmallCoarsenItems; ++i) {
-            const int64_t r = int64_t(tid) * kSmallCoarsenItems + i;
-            if (r < n) out[r] = v[i];
+    for (int i = 0; i < kSmallCoarsenItems; ++i) {
+        if (i >= items) break;
+        const unsigned long long upto = warp_scan(v[i]);
+        v[i] = mine + upto - v[i];
+        mine += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    unsigned long long total;
+    const unsigned long long base = warps_before(mine, totals, &total);
+#pragma unroll
+    for (int i = 0; i < kSmallCoarsenItems; ++i) {
+        const int r = first + 32 * i;
+        if (i < items && r < int(n)) {
+            sa[r] = int32_t(unsigned(base + v[i]));
+            sb[r] = int32_t((base + v[i]) >> 32);
         }
-        __syncthreads();  // the temp storage is reused
     }
 }
 
@@ -1201,11 +1264,11 @@ amdg_status device_transform_topology(amdg_grid* g, const DeviceTopoOut& out, in
     // counts of the vol rows in d_cnt[0 .. rows], of the flx rows in d_cnt[rows + 1 ..]
     int32_t* vcnt = d_cnt;
     int32_t* fcnt = d_cnt + rows + 1;
-    topo_count_kernel<<<blocks_for(32 * (rows + 1), 256), 256, 0, st>>>(A, vcnt, fcnt, out.long_count);
-    AMDG_CK(cudaGetLastError());
+    AMDG_CK(launch_after(topo_count_kernel, dim3(blocks_for(32 * (rows + 1), 256)), 256, 0, st, A, vcnt, fcnt,
+                         out.long_count));
     if (rows + 1 <= kSmallCoarsenMax) {
-        scan_pair_small_kernel<<<1, kSmallCoarsenThreads, 0, st>>>(vcnt, fcnt, rows + 1, out.vol_ptr, out.flx_ptr);
-        AMDG_CK(cudaGetLastError());
+        AMDG_CK(launch_after(scan_pair_small_kernel, dim3(1), kSmallCoarsenThreads, 0, st, vcnt, fcnt, rows + 1,
+                             out.vol_ptr, out.flx_ptr));
     } else {
         size_t temp = 0;
         AMDG_CK(cub::DeviceScan::ExclusiveSum(nullptr, temp, vcnt, out.vol_ptr, int(rows + 1), st));
@@ -1215,13 +1278,12 @@ amdg_status device_transform_topology(amdg_grid* g, const DeviceTopoOut& out, in
         tb = g->dev.temp_bytes;
         AMDG_CK(cub::DeviceScan::ExclusiveSum(g->dev.temp, tb, fcnt, out.flx_ptr, int(rows + 1), st));
     }
-    topo_fill_kernel<<<blocks_for(32 * rows, 256), 256, 0, st>>>(
-        A, out.vol_ptr, out.flx_ptr, reinterpret_cast<int2*>(out.vol_nbr), reinterpret_cast<int2*>(out.flx_nbr),
-        out.vol_split, out.flx_split, out.vol_cap, out.flx_cap, out.err, static_cast<RowRec*>(out.rows), out.long_count,
-        out.long_rows, out.long_stride);
-    AMDG_CK(cudaGetLastError());
-    ancestors_kernel<<<blocks_for(rows, 128), 128, 0, st>>>(A, out.anc_order, out.p1, out.anc, out.err);
-    AMDG_CK(cudaGetLastError());
+    AMDG_CK(launch_after(topo_fill_kernel, dim3(blocks_for(32 * rows, 256)), 256, 0, st, A, out.vol_ptr, out.flx_ptr,
+                         reinterpret_cast<int2*>(out.vol_nbr), reinterpret_cast<int2*>(out.flx_nbr), out.vol_split,
+                         out.flx_split, out.vol_cap, out.flx_cap, out.err, static_cast<RowRec*>(out.rows),
+                         out.long_count, out.long_rows, out.long_stride));
+    AMDG_CK(launch_after(ancestors_kernel, dim3(blocks_for(rows * out.p1, 128)), 128, 0, st, A, out.anc_order, out.p1,
+                         out.anc, out.err));
     g->ctx->launches += 6;
     return AMDG_OK;
 }

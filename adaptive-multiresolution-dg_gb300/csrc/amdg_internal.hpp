@@ -332,7 +332,7 @@ struct GridDevice {
     uint64_t* key_alt = nullptr;     // the next element set is assembled here, then swapped in
     int64_t key_cap = 0;
     unsigned long long* hkey = nullptr;  // hash slots (all bits set: empty)
-    int32_t* hval = nullptr;         // element index of the slot's key (-1: a key added by refinement)
+    int32_t* hval = nullptr;         // element index of the slot's key (-1: a key added by refinement); in hkey's allocation
     int64_t hcap = 0;                // slots (a power of two)
     int hbits = 0;
     int64_t hash_version = -1;       // element set the hash holds

@@ -676,7 +676,6 @@ amdg_status amdg_grid_destroy(amdg_grid* g) {
     cudaFree(d.key);
     cudaFree(d.key_alt);
     cudaFree(d.hkey);
-    cudaFree(d.hval);
     cudaFree(d.newk);
     cudaFree(d.flag);
     cudaFree(d.force);
