@@ -182,7 +182,7 @@ amdg_status batch_step(amdg_batch* b, amdg_precision prec, cudaStream_t st) {
             L.us = in[stage]; L.xs = sh[stage]; L.un = b->d_u; L.out = out[stage]; L.shadow_out = sh[sout[stage]];
             L.row_ptr = b->d_row_ptr; L.src = b->d_src; L.blk = b->d_blk; L.blocks = b->d_blocks32;
             L.pairs = reinterpret_cast<const int2*>(b->d_pairs); L.blocks_p = b->d_blocks32p;
-            L.coef = b->d_coef32; L.dt = b->d_dt; L.solve_of = b->d_solve;
+            L.coef = b->d_coef32; L.dt = b->d_dt; L.solve_of = b->d_solve; L.sms = b->sms;
             AMDG_CK(launch_batch<float, float>(L, st));
         } else {
             BatchLaunch<double, double> L{};
@@ -329,7 +329,7 @@ amdg_status autotune_batch(amdg_batch* b, cudaStream_t st) {
                     L.us = b->d_u; L.xs = hi_of(b, 0); L.un = b->d_u; L.out = b->d_u1; L.shadow_out = hi_of(b, 1);
                     L.row_ptr = b->d_row_ptr; L.src = b->d_src; L.blk = b->d_blk; L.blocks = b->d_blocks32;
                     L.pairs = reinterpret_cast<const int2*>(b->d_pairs); L.blocks_p = b->d_blocks32p;
-                    L.coef = b->d_coef32; L.dt = b->d_dt; L.solve_of = b->d_solve;
+                    L.coef = b->d_coef32; L.dt = b->d_dt; L.solve_of = b->d_solve; L.sms = b->sms;
                     if (e == cudaSuccess) e = launch_batch<float, float>(L, st);
                 } else {
                     BatchLaunch<double, double> L{};

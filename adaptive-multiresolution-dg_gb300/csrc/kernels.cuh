@@ -90,7 +90,7 @@ struct BatchLaunch {
     // order); 2 persistent, tiles taken from the counter `queue` (zero before the launch)
     int schedule;
     unsigned long long* queue;
-    int sms;  // multiprocessors of the device (persistent grids)
+    int sms;  // multiprocessors of the device (persistent grids; columns per thread, T = float)
 };
 template <typename T, typename X>
 cudaError_t launch_batch(const BatchLaunch<T, X>& L, cudaStream_t st);

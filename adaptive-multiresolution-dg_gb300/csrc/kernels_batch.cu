@@ -3,10 +3,11 @@
 // stage advances all of them.  Each element carries its solve index; the
 // solve's velocity c scales the per-dimension sum of the shared 1D blocks
 // (u_vx + upwind flux, one table per flux side), and the solve's dt enters
-// the fused SSP-RK3 epilogue.  Column layout as linear_col_kernel; the CTA
-// size TH (the tile: TH / np^(dim-1) elements per CTA) is a template
-// parameter the batch's autotuner picks (64 to 1024 threads for dim <= 3,
-// 256 above), beside the bulk-copy ring kernel of kernels.cu.
+// the fused SSP-RK3 epilogue.  Column layout as linear_col_kernel, one or np
+// columns per thread; the CTA size TH (the tile: TH / np^(dim-1) elements per
+// CTA, np times as many with np columns) is a template parameter the batch's
+// autotuner picks (64 to 1024 threads for dim <= 3, 256 above), beside the
+// bulk-copy ring kernel of kernels.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,14 +41,21 @@ __device__ __forceinline__ void load_padded_block(const T* p, T (&v)[BS]) {
     for (int i = 0; i < BS; ++i) v[i] = wt[i];
 }
 
-// One tile: G elements, (element, column) per thread, into the shared output block y
-template <int D, int NP, int TH, typename T, typename X>
+// Shape of a tile: NC neighbouring columns of one element per thread, G elements per CTA.
+template <int D, int NP, int TH, int NC>
+struct ColShape {
+    static constexpr int B = BPow<NP, D>::v;
+    static constexpr int P = B / NP / NC;                 // threads per element
+    static constexpr int G = TH / P > 0 ? TH / P : 1;     // launch_batch only launches TH >= B / NP
+};
+
+// One tile: G elements, NC columns of an element per thread, into the shared output block y
+template <int D, int NP, int TH, int NC, typename T, typename X>
 __device__ __forceinline__ void col_tile(const BatchLaunch<T, X>& L, int64_t tile, T* y) {
-    constexpr int B = BPow<NP, D>::v;
-    constexpr int C = B / NP;
-    constexpr int G = TH / C > 0 ? TH / C : 1;  // launch_batch only launches TH >= C
+    using S = ColShape<D, NP, TH, NC>;
+    constexpr int B = S::B, P = S::P, G = S::G;
     const int tid = threadIdx.x;
-    const int g = tid / C, c = tid - (tid / C) * C;
+    const int g = tid / P, c = (tid - g * P) * NC;  // the thread's first column
     const int64_t e = tile * G + g;
     const bool active = (g < G) && (e < L.num_elements);
     const int solve = active ? __ldg(L.solve_of + e) : 0;
@@ -60,12 +68,15 @@ __device__ __forceinline__ void col_tile(const BatchLaunch<T, X>& L, int64_t til
         for (int s = t + 1; s < D; ++s) stride *= NP;
         const int lo = c % stride, hi = c / stride;
         const int base = hi * stride * NP + lo;
+        const int step = t == D - 1 ? NP : 1;  // from a column to the next (stride is a multiple of NC but for t = D - 1)
         if (active) {
             const T ct = L.coef[solve * D + t];
             const T* table = L.blocks + (ct >= T(0) ? 0 : size_t(L.num_blocks) * NP * NP);
-            T acc[NP];
+            T acc[NC][NP];
 #pragma unroll
-            for (int q = 0; q < NP; ++q) acc[q] = T(0);
+            for (int u = 0; u < NC; ++u)
+#pragma unroll
+                for (int q = 0; q < NP; ++q) acc[u][q] = T(0);
             const int64_t beg = __ldg(L.row_ptr + e * D + t);
             const int64_t end = __ldg(L.row_ptr + e * D + t + 1);
             if (L.pairs && L.blocks_p) {
@@ -77,31 +88,38 @@ __device__ __forceinline__ void col_tile(const BatchLaunch<T, X>& L, int64_t til
                     T mv[BS];
                     load_padded_block<T, BS>(tab + size_t(pr.y) * BS, mv);
                     const X* x = L.xs + int64_t(pr.x) * B + base;
-                    T xv[NP];
+                    T xv[NC][NP];
 #pragma unroll
-                    for (int p = 0; p < NP; ++p) xv[p] = T(__ldg(x + p * stride));
+                    for (int u = 0; u < NC; ++u)
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) xv[u][p] = T(__ldg(x + u * step + p * stride));
 #pragma unroll
                     for (int p = 0; p < NP; ++p)
 #pragma unroll
-                        for (int q = 0; q < NP; ++q) acc[q] = fma(mv[p * NP + q], xv[p], acc[q]);
+                        for (int u = 0; u < NC; ++u)
+#pragma unroll
+                            for (int q = 0; q < NP; ++q) acc[u][q] = fma(mv[p * NP + q], xv[u][p], acc[u][q]);
                 }
             } else {
                 for (int64_t i = beg; i < end; ++i) {
                     const int64_t sidx = __ldg(L.src + i);
                     const T* m = table + __ldg(L.blk + i) * NP * NP;
                     const X* x = L.xs + sidx * B + base;
-                    T xv[NP];
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) xv[p] = T(__ldg(x + p * stride));
 #pragma unroll
                     for (int p = 0; p < NP; ++p)
 #pragma unroll
-                        for (int q = 0; q < NP; ++q) acc[q] = fma(__ldg(m + p * NP + q), xv[p], acc[q]);
+                        for (int u = 0; u < NC; ++u) {
+                            const T xv = T(__ldg(x + u * step + p * stride));
+#pragma unroll
+                            for (int q = 0; q < NP; ++q) acc[u][q] = fma(__ldg(m + p * NP + q), xv, acc[u][q]);
+                        }
                 }
             }
             T* yb = y + g * B + base;
 #pragma unroll
-            for (int q = 0; q < NP; ++q) yb[q * stride] += ct * acc[q];
+            for (int u = 0; u < NC; ++u)
+#pragma unroll
+                for (int q = 0; q < NP; ++q) yb[u * step + q * stride] += ct * acc[u][q];
         }
         __syncthreads();
     }
@@ -129,14 +147,12 @@ __device__ __forceinline__ void col_tile(const BatchLaunch<T, X>& L, int64_t til
 // SCHED 0: one CTA per tile; 1: persistent, a grid of resident CTAs, CTA b takes tiles b, b + grid,
 // ...; 2: persistent, tiles taken one at a time from the device counter L.queue (zeroed before
 // the launch).  Each tile is computed alike, so the three give identical results.
-template <int D, int NP, int TH, typename T, typename X, int SCHED>
+template <int D, int NP, int TH, int NC, typename T, typename X, int SCHED>
 __global__ void __launch_bounds__(TH) batch_col_kernel(BatchLaunch<T, X> L) {
-    constexpr int B = BPow<NP, D>::v;
-    constexpr int C = B / NP;
-    constexpr int G = TH / C > 0 ? TH / C : 1;
-    __shared__ T y[G * B];
+    constexpr int G = ColShape<D, NP, TH, NC>::G;
+    __shared__ T y[G * ColShape<D, NP, TH, NC>::B];
     if constexpr (SCHED == 0) {
-        col_tile<D, NP, TH, T, X>(L, blockIdx.x, y);
+        col_tile<D, NP, TH, NC, T, X>(L, blockIdx.x, y);
     } else {
         const int64_t ntiles = (L.num_elements + G - 1) / G;
         __shared__ long long next;
@@ -147,7 +163,7 @@ __global__ void __launch_bounds__(TH) batch_col_kernel(BatchLaunch<T, X> L) {
             tile = next;
         }
         while (tile < ntiles) {
-            col_tile<D, NP, TH, T, X>(L, tile, y);
+            col_tile<D, NP, TH, NC, T, X>(L, tile, y);
             __syncthreads();  // y and `next` are reused by the next tile
             if constexpr (SCHED == 1) {
                 tile += gridDim.x;
@@ -170,30 +186,50 @@ bool batch_tile_supported(int dim, int np, int threads) {
 
 // resident CTAs per multiprocessor of a persistent schedule, queried once per kernel (the first
 // query runs when the batch is built, before any stream capture: batch_prepare_persistent)
-template <int D, int NP, int TH, typename T, typename X, int SCHED>
+template <int D, int NP, int TH, int NC, typename T, typename X, int SCHED>
 int col_per_sm() {
     static int per_sm = 0;
     if (per_sm == 0 &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_col_kernel<D, NP, TH, T, X, SCHED>, TH, 0) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_col_kernel<D, NP, TH, NC, T, X, SCHED>, TH, 0) !=
             cudaSuccess)
         per_sm = 0;
     return per_sm;
 }
 
-template <int D, int NP, int TH, typename T, typename X, int SCHED>
-cudaError_t launch_col_sched(const BatchLaunch<T, X>& L, cudaStream_t st, bool prepare_only) {
-    constexpr int C = BPow<NP, D>::v / NP;
-    constexpr int G = TH / C > 0 ? TH / C : 1;
+template <int D, int NP, int TH, int NC, typename T, typename X, int SCHED>
+cudaError_t launch_col(const BatchLaunch<T, X>& L, cudaStream_t st, bool prepare_only) {
+    constexpr int G = ColShape<D, NP, TH, NC>::G;
     int64_t grid = (L.num_elements + G - 1) / G;
     if (SCHED != 0) {
-        const int per_sm = col_per_sm<D, NP, TH, T, X, SCHED>();
+        const int per_sm = col_per_sm<D, NP, TH, NC, T, X, SCHED>();
         if (per_sm <= 0) return cudaErrorInvalidConfiguration;
         grid = std::max<int64_t>(1, std::min<int64_t>(grid, int64_t(per_sm) * std::max(L.sms, 1)));
         if (SCHED == 2 && !L.queue && !prepare_only) return cudaErrorInvalidValue;
     }
     if (prepare_only) return cudaSuccess;
-    batch_col_kernel<D, NP, TH, T, X, SCHED><<<unsigned(grid), TH, 0, st>>>(L);
+    batch_col_kernel<D, NP, TH, NC, T, X, SCHED><<<unsigned(grid), TH, 0, st>>>(L);
     return cudaGetLastError();
+}
+
+// Columns per thread.  A thread with one column reads np^2 + np values per neighbour for its np^2
+// multiply-adds, and the 16-byte reads of the 1D block, the same for all columns of an element, take
+// most of the L1 cache's cycles (85 % of its rate at 198,432 elements, 3D, np = 3).  With np
+// neighbouring columns per thread the block is read by np times fewer threads: 0.145 -> 0.132 ms per
+// stage there, 0.108 -> 0.087 at 59,616 elements in 4D, 0.090 -> 0.077 at 19,902 in 5D.  np = 3 only: with
+// np = 4 the wider spread of a warp's reads costs more (99,760 elements, 3D: 0.143 -> 0.225), with
+// np = 2 nothing is gained (298,496: 0.068 -> 0.073).  And it takes kMultiColumnThreads
+// threads per multiprocessor: 59,840 elements in 3D gain (0.041 -> 0.038), 19,968 lose (0.018 -> 0.022).
+constexpr int kMultiColumnThreads = 1024;
+template <int D, int NP, int TH, typename T, typename X, int SCHED>
+cudaError_t launch_col_sched(const BatchLaunch<T, X>& L, cudaStream_t st, bool prepare_only) {
+    if constexpr (NP == 3 && D >= 3 && std::is_same<T, float>::value) {
+        const int64_t threads = L.num_elements * ColShape<D, NP, TH, NP>::P;
+        if (prepare_only || threads >= int64_t(kMultiColumnThreads) * std::max(L.sms, 1)) {
+            const cudaError_t e = launch_col<D, NP, TH, NP, T, X, SCHED>(L, st, prepare_only);
+            if (!prepare_only || e != cudaSuccess) return e;
+        }
+    }
+    return launch_col<D, NP, TH, 1, T, X, SCHED>(L, st, prepare_only);
 }
 
 template <int D, int NP, int TH, typename T, typename X>
