@@ -574,6 +574,8 @@ struct TopoArgs {
     int64_t E;
     KeyShape ks;
     KeyHash h;
+    const uint8_t* seen;  // [order][n1]
+    int n1;
 };
 
 // The candidate 1D orders of level l for a row (element, dimension t) with 1D support [a0, b0),
@@ -618,7 +620,8 @@ __device__ __forceinline__ int cand_order(const LevelCands& c, int i) {
 // One warp per row (element, dimension): the candidates of all levels in one sequence, looked up 32 at a
 // time, the present ones counted (out == nullptr) or written in order (ballot prefix).  Returns the
 // vol / flx counts and the counts at levels up to the element's own (the split between the "U" and
-// "L" parts).  Most rows have a few candidates on each level: taken level by level, a row waited
+// "L" parts).  The finer vol neighbours without a point of the element are written from the end
+// of the list down (RowRec in kernels_plan.cuh); *skip_out is their number.  Most rows have a few candidates on each level: taken level by level, a row waited
 // for nmax + 1 lookups one after the other (the fill 32 us at 3,880 elements in two dimensions, cold
 // caches, 14 us at 390; 22 and 10 us with the levels in one sequence).
 struct RowOut {
@@ -627,14 +630,14 @@ struct RowOut {
     int64_t vmax, fmax;  // entries the row may write (fill)
 };
 __device__ __forceinline__ void row_lists(const TopoArgs& A, int64_t e, int t, const RowOut* out, int* nv_out,
-                                          int* nf_out, int* sv_out, int* sf_out) {
+                                          int* nf_out, int* sv_out, int* sf_out, int* skip_out) {
     const int lane = threadIdx.x & 31;
     const int nmax = A.ks.nmax;
     const uint64_t key = A.keys[e];
     const int oi = A.ks.field(key, t), own = level_of(oi);
     int64_t a0, b0;
     support_of(oi, nmax, &a0, &b0);
-    int nv = 0, nf = 0, sv = 0, sf = 0;
+    int nv = 0, nf = 0, sv = 0, sf = 0, skip = 0;
     // lane l holds the number of candidates up to level l; those of the "U" part come first
     const int upto = warp_scan(lane <= nmax ? level_cands(lane, nmax, a0, b0).n : 0);
     const int total = __shfl_sync(0xffffffffu, upto, nmax), upper = __shfl_sync(0xffffffffu, upto, own);
@@ -664,10 +667,13 @@ __device__ __forceinline__ void row_lists(const TopoArgs& A, int64_t e, int t, c
                 const int pf = nf + __popc(bf & below);
                 if (pf < out->fmax) out->flx[pf] = make_int2(s, o);
             }
+            const bool last = inv && i >= upper && !A.seen[int64_t(oi) * A.n1 + o];
+            const unsigned bs = __ballot_sync(0xffffffffu, last);
             if (inv) {
-                const int pv = nv + __popc(bv & below);
-                if (pv < out->vmax) out->vol[pv] = make_int2(s, o);
+                const int64_t pv = last ? out->vmax - 1 - (skip + __popc(bs & below)) : nv - skip + __popc(bv & ~bs & below);
+                if (pv >= 0 && pv < out->vmax) out->vol[pv] = make_int2(s, o);
             }
+            skip += __popc(bs);
         }
         nf += __popc(bf);
         nv += __popc(bv);
@@ -680,6 +686,7 @@ __device__ __forceinline__ void row_lists(const TopoArgs& A, int64_t e, int t, c
     *nf_out = nf;
     *sv_out = sv;
     *sf_out = sf;
+    *skip_out = skip;
 }
 
 __global__ void topo_count_kernel(TopoArgs A, int32_t* vcnt, int32_t* fcnt, int32_t* long_count) {
@@ -693,8 +700,8 @@ __global__ void topo_count_kernel(TopoArgs A, int32_t* vcnt, int32_t* fcnt, int3
         return;
     }
     const int64_t e = row / dim;
-    int nv, nf, sv, sf;
-    row_lists(A, e, int(row - e * dim), nullptr, &nv, &nf, &sv, &sf);
+    int nv, nf, sv, sf, skip;
+    row_lists(A, e, int(row - e * dim), nullptr, &nv, &nf, &sv, &sf, &skip);
     if ((threadIdx.x & 31) == 0) {
         vcnt[row] = nv;
         fcnt[row] = nf;
@@ -716,20 +723,20 @@ __global__ void topo_fill_kernel(TopoArgs A, const int32_t* vol_ptr, const int32
         if ((threadIdx.x & 31) == 0) {
             atomicOr(err, 1);
             const int o = A.ks.field(A.keys[row / dim], int(row % dim));
-            write_row_rec(rows, row, dim, 0, 0, 0, 0, 0, 0, o, long_count, long_rows, long_stride);
+            write_row_rec(rows, row, dim, 0, 0, 0, 0, 0, 0, o, 0, long_count, long_rows, long_stride);
         }
         return;
     }
     const RowOut out{vol_nbr + v0, flx_nbr + f0, v1 - v0, f1 - f0};
     const int64_t e = row / dim;
-    int nv, nf, sv, sf;
-    row_lists(A, e, int(row - e * dim), &out, &nv, &nf, &sv, &sf);
+    int nv, nf, sv, sf, skip;
+    row_lists(A, e, int(row - e * dim), &out, &nv, &nf, &sv, &sf, &skip);
     if ((threadIdx.x & 31) == 0) {
         if (nv != v1 - v0 || nf != f1 - f0) atomicOr(err, 1);
         vol_split[row] = int32_t(v0 + sv);
         flx_split[row] = int32_t(f0 + sf);
         write_row_rec(rows, row, dim, int(v0), int(v0 + sv), int(v1), int(f0), int(f0 + sf), int(f1),
-                      A.ks.field(A.keys[e], int(row - e * dim)), long_count, long_rows, long_stride);
+                      A.ks.field(A.keys[e], int(row - e * dim)), skip, long_count, long_rows, long_stride);
     }
 }
 
@@ -1260,7 +1267,7 @@ amdg_status device_transform_topology(amdg_grid* g, const DeviceTopoOut& out, in
     const int64_t E = g->host.num_elements;
     const int dim = g->host.dim;
     const int64_t rows = E * dim;
-    TopoArgs A{g->dev.key, E, KeyShape{dim, g->host.nmax}, hash_of(g)};
+    TopoArgs A{g->dev.key, E, KeyShape{dim, g->host.nmax}, hash_of(g), out.seen, out.n1};
     // counts of the vol rows in d_cnt[0 .. rows], of the flx rows in d_cnt[rows + 1 ..]
     int32_t* vcnt = d_cnt;
     int32_t* fcnt = d_cnt + rows + 1;
@@ -1293,7 +1300,7 @@ amdg_status device_parent_table(amdg_grid* g, int32_t* d_pg, void* stream) {
     const int64_t E = g->host.num_elements;
     const int dim = g->host.dim;
     if (E == 0) return AMDG_OK;
-    TopoArgs A{g->dev.key, E, KeyShape{dim, g->host.nmax}, hash_of(g)};
+    TopoArgs A{g->dev.key, E, KeyShape{dim, g->host.nmax}, hash_of(g), nullptr, 0};
     parent_table_kernel<<<blocks_for(E * dim, 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(A, d_pg);
     AMDG_CK(cudaGetLastError());
     g->ctx->launches++;

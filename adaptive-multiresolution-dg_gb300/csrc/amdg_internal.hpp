@@ -513,6 +513,8 @@ struct amdg_burgers_op {
     double *d_u1 = nullptr, *d_u2 = nullptr, *d_rhs64 = nullptr, *d_pred = nullptr;
     std::vector<double> host_norms;
     // one SSP-RK3 step captured as a CUDA graph, valid for (grid version, precision, dt)
+    std::vector<uint8_t> seen;       // [order][n1]: the interval of the second order holds a point of the first
+    uint8_t* d_seen = nullptr;
     int32_t* d_anc_order = nullptr;  // device copy of anc_order (the device-built ancestors)
     int32_t* d_topo_cnt = nullptr;   // per (element, dimension) list lengths of the device build
     unsigned long long* d_cls = nullptr;  // learned step: [refined by the network, unsure] (device)
@@ -599,6 +601,8 @@ struct DeviceTopoOut {
     void* rows;                      // RowRec per (element, dimension) (kernels_plan.cuh)
     int32_t *long_count, *long_rows; // long rows per dimension: counts, elements [dim][long_stride]
     int64_t long_stride;
+    const uint8_t* seen;             // [order][n1]: whether the interval of the second order holds points of the first
+    int n1;
 };
 // bounds on the number of (element, neighbour) pairs of the vol and flx lists over all dimensions
 void transform_topology_bounds(const amdg_grid* g, int64_t* vol_pairs, int64_t* flx_pairs);

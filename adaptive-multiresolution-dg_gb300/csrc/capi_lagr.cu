@@ -894,12 +894,43 @@ amdg_status device_topology(amdg_burgers_op* op, cudaStream_t st) {
     const size_t fcap = op->dev_cap[static_cast<const void*>(&op->d_flx_nbr)] / (2 * sizeof(int32_t));
     DeviceTopoOut out{op->d_vol_ptr, op->d_vol_nbr, op->d_vol_split, op->d_flx_ptr, op->d_flx_nbr, op->d_flx_split,
                       op->d_anc, int64_t(vcap), int64_t(fcap), op->d_anc_order, op->p1, err,
-                      op->d_rows, op->d_long, op->d_long + kMaxDim, op->long_stride};
+                      op->d_rows, op->d_long, op->d_long + kMaxDim, op->long_stride, op->d_seen, op->n1};
     if ((s = device_transform_topology(g, out, op->d_topo_cnt, st)) != AMDG_OK) return s;
     // a set that came from the host may have holes: report them now (sets the device refine and
     // coarsen produce are hole-free; their build errors surface at the next element-set change)
     if (!g->host_stale) return grid_check_topology(g);
     return AMDG_OK;
+}
+
+// Host-built lists in the device builder's order: of a row's finer vol neighbours those that hold one
+// of the element's interpolation points first, the others (skip: their number) from the end down.
+void points_first(const amdg_burgers_op* op, TransformTopology* topo, std::vector<int32_t>* skip) {
+    const HostGrid& h = op->grid->host;
+    const int64_t rows = h.num_elements * h.dim;
+    skip->assign(size_t(rows), 0);
+    std::vector<std::pair<int32_t, int32_t>> rest;
+    for (int64_t r = 0; r < rows; ++r) {
+        const uint8_t* seen = &op->seen[size_t(h.order[size_t(r)]) * op->n1];
+        int32_t* nbr = topo->vol_nbr.data();
+        const int32_t end = topo->vol_ptr[size_t(r) + 1];
+        int32_t at = topo->vol_split[size_t(r)];
+        rest.clear();
+        for (int32_t i = at; i < end; ++i) {
+            const int32_t s = nbr[2 * size_t(i)], o = nbr[2 * size_t(i) + 1];
+            if (!seen[o]) {
+                rest.push_back({s, o});
+                continue;
+            }
+            nbr[2 * size_t(at)] = s;
+            nbr[2 * size_t(at) + 1] = o;
+            ++at;
+        }
+        for (size_t q = 0; q < rest.size(); ++q) {
+            nbr[2 * (size_t(end) - 1 - q)] = rest[q].first;
+            nbr[2 * (size_t(end) - 1 - q) + 1] = rest[q].second;
+        }
+        (*skip)[size_t(r)] = int32_t(rest.size());
+    }
 }
 
 // (Re)build the neighbour lists and surplus ancestors for the grid's current
@@ -926,7 +957,8 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
         if ((s = grid_ensure_host(g)) != AMDG_OK) return s;
         TransformTopology topo;
         build_transform_topology(g->host, &topo);
-        std::vector<int32_t> anc;
+        std::vector<int32_t> anc, vol_skip;
+        points_first(op, &topo, &vol_skip);
         if (!build_surplus_ancestors(g->host, t, &anc))
             return fail(AMDG_ERR_STATE, "element set has a hole: a surplus ancestor is missing");
         if ((s = upload_grow(op, &op->d_vol_ptr, topo.vol_ptr, st)) != AMDG_OK ||
@@ -938,7 +970,9 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
             (s = upload_grow(op, &op->d_flx_split, topo.flx_split, st)) != AMDG_OK || (s = reserve_rows(op)) != AMDG_OK)
             return s;
         AMDG_CK(cudaMemsetAsync(op->d_long, 0, kMaxDim * sizeof(int32_t), st));
-        AMDG_CK(launch_pack_rows(op->d_vol_ptr, op->d_vol_split, op->d_flx_ptr, op->d_flx_split, g->d_order,
+        // the skip counts are only needed for the records: they go through the device builder's count scratch
+        if ((s = upload_grow(op, &op->d_topo_cnt, vol_skip, st)) != AMDG_OK) return s;
+        AMDG_CK(launch_pack_rows(op->d_vol_ptr, op->d_vol_split, op->d_topo_cnt, op->d_flx_ptr, op->d_flx_split, g->d_order,
                                  g->host.num_elements, g->host.dim, static_cast<RowRec*>(op->d_rows), op->d_long,
                                  op->d_long + kMaxDim, op->long_stride, st));
         g->ctx->launches++;
@@ -1075,6 +1109,16 @@ static amdg_status lagr_create(amdg_grid* g, int kind, const double* alpha, doub
         delete op;
         return fail(AMDG_ERR_ARG, "Lagrange table of unexpected size");
     }
+    // which intervals hold points of which: the nonzero blocks of the transforms to point values
+    op->seen.assign(size_t(op->n1) * op->n1, 0);
+    for (int from = 0; from < op->n1; ++from)
+        for (int to = 0; to < op->n1; ++to) {
+            const size_t block = size_t(np) * op->p1, at = (size_t(from) * op->n1 + to) * block;
+            bool any = false;
+            for (size_t q = at; q < at + block && !any; ++q)
+                any = t.a2p[q] != 0.0 || (kind == 1 && t.a2pd[q] != 0.0);
+            op->seen[size_t(to) * op->n1 + from] = any ? 1 : 0;
+        }
     std::memcpy(op->weight, t.weight, sizeof(op->weight));
     transform_schedule(dim, &op->sched_dims, &op->sched_lu);
     build_terms(op);
@@ -1095,7 +1139,8 @@ static amdg_status lagr_create(amdg_grid* g, int kind, const double* alpha, doub
                        (s = upload_vec(&op->d_pts, t.pts)) != AMDG_OK || (s = point_sines()) != AMDG_OK)) ||
         (s = upload_df(&op->df_a2p, t.a2p)) != AMDG_OK || (kind == 1 && (s = upload_df(&op->df_a2pd, t.a2pd)) != AMDG_OK) ||
         (s = upload_vec(&op->d_anc_point, t.anc_point)) != AMDG_OK || (s = upload_vec(&op->d_anc_rank, t.anc_rank)) != AMDG_OK ||
-        (s = upload_vec(&op->d_terms, op->terms)) != AMDG_OK || (s = burgers_sync(op)) != AMDG_OK) {
+        (s = upload_vec(&op->d_terms, op->terms)) != AMDG_OK || (s = upload_vec(&op->d_seen, op->seen)) != AMDG_OK ||
+        (s = burgers_sync(op)) != AMDG_OK) {
         amdg_burgers_destroy(op);
         return s;
     }
@@ -1129,7 +1174,7 @@ amdg_status amdg_burgers_destroy(amdg_burgers_op* op) {
                     op->d_feat, op->d_prob, op->d_a2pd, op->d_ljv, op->d_pts, op->f_a2pd, op->f_ljv,
                     op->w_fields, op->d_v1, op->d_su, op->d_sv, op->df_a2p, op->df_a2pd,
                     op->d_anc_order, op->d_topo_cnt, op->d_cls, op->d_nodes, op->d_plan_nodes, op->d_plan_products,
-                    op->d_rows, op->d_long, op->d_sines};
+                    op->d_rows, op->d_long, op->d_sines, op->d_seen};
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(op->h_cls);
     delete op;
@@ -1162,13 +1207,15 @@ amdg_status amdg_burgers_work(amdg_burgers_op* op, double* flops, double* transf
         AMDG_CK(cudaMemcpy(ptr[f].data(), dp[f], size_t(rows + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost));
         if (rows) AMDG_CK(cudaMemcpy(split[f].data(), ds[f], size_t(rows) * sizeof(int32_t), cudaMemcpyDeviceToHost));
     }
-    double cnt[kMaxDim][2][3] = {};
+    std::vector<RowRec> recs(static_cast<size_t>(rows));
+    if (rows) AMDG_CK(cudaMemcpy(recs.data(), op->d_rows, size_t(rows) * sizeof(RowRec), cudaMemcpyDeviceToHost));
+    double cnt[kMaxDim][3][3] = {};  // lists: vol, flx, vol of the planned transforms to point values
     for (int64_t r = 0; r < rows; ++r)
-        for (int f = 0; f < 2; ++f) {
-            const int t = int(r % dim);
-            cnt[t][f][0] += ptr[f][r + 1] - split[f][r];  // "L": finer neighbours
-            cnt[t][f][1] += ptr[f][r + 1] - ptr[f][r];
-            cnt[t][f][2] += split[f][r] - ptr[f][r];      // "U": coarser or equal
+        for (int f = 0; f < 3; ++f) {
+            const int t = int(r % dim), q = f == 1 ? 1 : 0, end = ptr[q][r + 1] - (f == 2 ? recs[size_t(r)].flx.w >> 1 : 0);
+            cnt[t][f][0] += end - split[q][r];  // "L": finer neighbours
+            cnt[t][f][1] += end - ptr[q][r];
+            cnt[t][f][2] += split[q][r] - ptr[q][r];  // "U": coarser or equal
         }
     // the sweeps one right-hand side runs: the products of its plans, or the nodes of its sweep trees
     double fl = 0.0, pairs = 0.0;
@@ -1205,7 +1252,8 @@ amdg_status amdg_burgers_work(amdg_burgers_op* op, double* flops, double* transf
                     const PlanNode& n = op->plan_nodes[size_t(plan.offset[j] + k)];
                     for (int q = 0; q < n.count; ++q) {
                         const PlanProduct& p = op->plan_products[size_t(n.first + q)];
-                        add(p.in < 0 ? -1 : j, p.t, p.flx, p.lu);
+                        const bool points = p.mat == kMatA2P || p.mat == kMatA2PD;
+                        add(p.in < 0 ? -1 : j, p.t, points ? 2 : p.flx, p.lu);
                     }
                 }
             continue;

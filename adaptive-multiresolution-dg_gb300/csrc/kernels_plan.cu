@@ -76,6 +76,7 @@ __device__ __forceinline__ Fibre<T> fibre_of(const PlanArgs<T>& a, const PlanPro
     f.nbr = D.flx ? a.flx_nbr : a.vol_nbr;
     f.beg = D.lu == 0 ? r.y : r.x;  // "L": neighbours finer than e along t; "U": coarser or equal
     f.end = D.lu == 2 ? r.y : r.z;
+    if (D.lu != 2 && (D.mat == kMatA2P || D.mat == kMatA2PD)) f.end -= __ldg(&row->flx.w) >> 1;  // zero blocks
     const bool pen = D.in < 0;
     f.nf = pen ? a.np : NF;
     f.in = pen ? a.pen_in : (a.first_sweep ? a.src[D.in] : a.in + int64_t(D.in) * a.in_slice);
@@ -264,7 +265,7 @@ __device__ __forceinline__ void fibre_column(const Fibre<T>& f, int c, T (&acc)[
 template <typename T>
 __device__ __forceinline__ bool long_row(const PlanArgs<T>& a, const PlanNode& node, int64_t e) {
     for (int t = 0; t < a.dim; ++t)
-        if ((node.long_mask >> t & 1) && __ldg(&a.rows[e * a.dim + t].flx.w)) return true;
+        if ((node.long_mask >> t & 1) && (__ldg(&a.rows[e * a.dim + t].flx.w) & 1)) return true;
     return false;
 }
 
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
                 const int64_t e = __ldg(a.long_rows + int64_t(t) * a.long_stride + (u - first_unit) / chunks);
                 bool earlier = false;  // listed under an earlier dimension too: done there
                 for (int s = 0; s < t; ++s)
-                    earlier = earlier || ((node.long_mask >> s & 1) && __ldg(&a.rows[e * a.dim + s].flx.w));
+                    earlier = earlier || ((node.long_mask >> s & 1) && (__ldg(&a.rows[e * a.dim + s].flx.w) & 1));
                 if (earlier) continue;
                 const int c0 = ((u - first_unit) % chunks) * kLongItems;
                 const int total = np * kLongItems;
@@ -632,22 +633,23 @@ template cudaError_t launch_plan_out<float>(const PlanArgs<float>&, const PlanOu
 template cudaError_t launch_plan_out<float2>(const PlanArgs<float2>&, const PlanOut&, cudaStream_t);
 
 __global__ void pack_rows_kernel(const int32_t* __restrict__ vol_ptr, const int32_t* __restrict__ vol_split,
+                                 const int32_t* __restrict__ vol_skip,
                                  const int32_t* __restrict__ flx_ptr, const int32_t* __restrict__ flx_split,
                                  const int32_t* __restrict__ order, int64_t num_rows, int dim, RowRec* __restrict__ rows,
                                  int32_t* long_count, int32_t* long_rows, int64_t long_stride) {
     const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= num_rows) return;
     write_row_rec(rows, r, dim, vol_ptr[r], vol_split[r], vol_ptr[r + 1], flx_ptr[r], flx_split[r], flx_ptr[r + 1], order[r],
-                  long_count, long_rows, long_stride);
+                  vol_skip[r], long_count, long_rows, long_stride);
 }
 
-cudaError_t launch_pack_rows(const int32_t* vol_ptr, const int32_t* vol_split, const int32_t* flx_ptr,
-                             const int32_t* flx_split, const int32_t* order, int64_t num_elements, int dim, RowRec* rows,
+cudaError_t launch_pack_rows(const int32_t* vol_ptr, const int32_t* vol_split, const int32_t* vol_skip,
+                             const int32_t* flx_ptr, const int32_t* flx_split, const int32_t* order, int64_t num_elements, int dim, RowRec* rows,
                              int32_t* long_count, int32_t* long_rows, int64_t long_stride, cudaStream_t st) {
     const int64_t n = num_elements * dim;
     if (n == 0) return cudaSuccess;
-    pack_rows_kernel<<<unsigned((n + 127) / 128), 128, 0, st>>>(vol_ptr, vol_split, flx_ptr, flx_split, order, n, dim, rows,
-                                                                long_count, long_rows, long_stride);
+    pack_rows_kernel<<<unsigned((n + 127) / 128), 128, 0, st>>>(vol_ptr, vol_split, vol_skip, flx_ptr, flx_split, order, n,
+                                                                dim, rows, long_count, long_rows, long_stride);
     return cudaGetLastError();
 }
 
