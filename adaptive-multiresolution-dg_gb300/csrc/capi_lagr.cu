@@ -400,9 +400,9 @@ SweepArgs<T> sweep_args(const amdg_burgers_op* op, const Mats<T>& m) {
     a.n1 = op->n1;
     a.num_elements = g->host.num_elements;
     a.desc = op->d_terms;
-    // default kernels (measured on the config-3 runs): warp per (node, element) for the FP32 sweeps
-    // (fewer issued instructions), thread per output entry for the FP64 ones (FP64-pipe work per
-    // warp kept whole) and the double-float ones (their arithmetic, not the issue overhead, binds)
+    // in one dimension (no plan): warp per (node, element) for the FP32 sweeps (fewer issued
+    // instructions), thread per output entry for the FP64 ones (FP64-pipe work per warp kept whole)
+    // and the double-float ones (their arithmetic, not the issue overhead, binds)
     a.variant = op->sweep_variant >= 0 ? op->sweep_variant : (std::is_same<T, float>::value ? 2 : 0);
     for (int i = 0; i < kNumLagrMats; ++i) a.mats[i] = m.m[i];
     a.vol_ptr = op->d_vol_ptr;
@@ -536,12 +536,13 @@ amdg_status eval_point_values(amdg_burgers_op* op, const Mats<T>& m, const T* u,
 
 // u_h at the interpolation points in double-float arithmetic (the mixed mode): the sweeps on the
 // FP32 pipe with about 48-bit precision, the slices summed in FP64 into up, or, when fp is
-// given, f(u) = u^2/2 at the points into fp
-amdg_status eval_point_values_df(amdg_burgers_op* op, const double* u, double* up, double* fp, cudaStream_t st) {
+// given, f(u) = u^2/2 at the points into fp; u32, when given, receives u in FP32
+amdg_status eval_point_values_df(amdg_burgers_op* op, const double* u, double* up, double* fp, cudaStream_t st,
+                                 float* u32 = nullptr) {
     const int np = op->grid->host.k + 1;
     const int64_t n = op->grid->host.num_elements * op->points;
     float2* udf = static_cast<float2*>(op->w_u);
-    AMDG_CK(launch_to_df(u, udf, op->grid->dof, st));
+    AMDG_CK(launch_to_df(u, udf, u32, op->grid->dof, st));
     op->grid->ctx->launches++;
     float2* slots = static_cast<float2*>(op->w_slots);
     const float2* src[1] = {udf};
@@ -673,7 +674,7 @@ amdg_status eval_wave_penalty(amdg_burgers_op* op, const double* u, double* rhs,
 // coefficients (type To) into fields dim+1 .. 2 dim+1 of w_fields
 template <typename To>
 amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, cudaStream_t st, int f_first = 0,
-                             int f_last = -1) {
+                             int f_last = -1, float* u32 = nullptr) {
     amdg_grid* g = op->grid;
     const int dim = g->host.dim, np = g->host.k + 1;
     const int64_t E = g->host.num_elements, n = E * op->points;
@@ -686,7 +687,7 @@ amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, c
     Tp* slots = static_cast<Tp*>(op->w_slots);
     const Tp* src[1];
     if constexpr (df) {
-        AMDG_CK(launch_to_df(u, static_cast<float2*>(op->w_u), g->dof, st));
+        AMDG_CK(launch_to_df(u, static_cast<float2*>(op->w_u), u32, g->dof, st));
         op->grid->ctx->launches++;
         src[0] = static_cast<const float2*>(op->w_u);
     } else {
@@ -775,6 +776,11 @@ void wave_field_coefs(amdg_burgers_op* op, To** fc) {
     for (int f = 0; f <= dim; ++f) fc[f] = reinterpret_cast<To*>(fields + size_t(dim + 1 + f) * stride);
 }
 
+// the FP32 state of a mixed right-hand side, behind the double-float one in w_u
+float* state32(amdg_burgers_op* op) {
+    return reinterpret_cast<float*>(static_cast<float2*>(op->w_u) + size_t(op->capacity) * op->grid->block);
+}
+
 // rhs (FP64, dof entries) of the FP64 state u, or the stage update `so` with it.
 // The point values and the hierarchical surplus always run in FP64:
 // fine-level surpluses are small differences of O(1) point values, which FP32
@@ -795,16 +801,14 @@ amdg_status eval_rhs(amdg_burgers_op* op, const double* u, double* rhs, amdg_pre
         }
         float* fc[kMaxTermSources];
         for (int f = 0; f <= dim; ++f) fc[f] = reinterpret_cast<float*>(fields + size_t(dim + 1 + f) * stride);
-        if (amdg_status r = eval_wave_fields<float>(op, u, fc, st); r != AMDG_OK) return r;
-        float* u32 = static_cast<float*>(op->w_u);
-        AMDG_CK(launch_convert<double, float>(u, u32, op->grid->dof, st));
-        op->grid->ctx->launches++;
+        float* u32 = state32(op);
+        if (amdg_status r = eval_wave_fields<float>(op, u, fc, st, 0, -1, u32); r != AMDG_OK) return r;
         return eval_back_transforms<float>(op, mats32(op), fc, dim + 1, u32, rhs, so, st);
     }
     double* fp = static_cast<double*>(op->w_a);
     amdg_status r = prec == AMDG_PREC_FP64
                         ? eval_point_values<double>(op, mats64(op), u, static_cast<double*>(op->w_up), fp, st)
-                        : eval_point_values_df(op, u, static_cast<double*>(op->w_up), fp, st);
+                        : eval_point_values_df(op, u, static_cast<double*>(op->w_up), fp, st, state32(op));
     if (r != AMDG_OK) return r;
     if (prec == AMDG_PREC_FP64) {
         double* fu = static_cast<double*>(op->w_fu);
@@ -813,12 +817,9 @@ amdg_status eval_rhs(amdg_burgers_op* op, const double* u, double* rhs, amdg_pre
         return eval_back_transforms<double>(op, mats64(op), src, 1, u, rhs, so, st);
     }
     float* fu32 = static_cast<float*>(op->w_fu);
-    float* u32 = static_cast<float*>(op->w_u);
     if ((r = eval_surplus<double, float>(op, fp, fu32, st)) != AMDG_OK) return r;
-    AMDG_CK(launch_convert<double, float>(u, u32, op->grid->dof, st));
-    op->grid->ctx->launches++;
     const float* src[1] = {fu32};
-    return eval_back_transforms<float>(op, mats32(op), src, 1, u32, rhs, so, st);
+    return eval_back_transforms<float>(op, mats32(op), src, 1, state32(op), rhs, so, st);
 }
 
 // Copy a host vector into a grow-only device array of the operator (stream
@@ -997,7 +998,7 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
         const size_t slices = size_t(op->chunk) * work;
         if ((s = alloc_bytes(&op->w_up, work)) != AMDG_OK || (s = alloc_bytes(&op->w_fu, work)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_a, work)) != AMDG_OK || (s = alloc_bytes(&op->w_b, work)) != AMDG_OK ||
-            (s = alloc_bytes(&op->w_u, vec)) != AMDG_OK || (s = alloc_bytes(&op->w_s0, slices)) != AMDG_OK ||
+            (s = alloc_bytes(&op->w_u, vec + vec / 2)) != AMDG_OK || (s = alloc_bytes(&op->w_s0, slices)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_s1, slices)) != AMDG_OK || (s = alloc_bytes(&op->w_slots, slices)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_u1), vec)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_u2), vec)) != AMDG_OK ||

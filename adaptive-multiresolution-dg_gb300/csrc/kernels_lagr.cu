@@ -4,7 +4,9 @@
 // dim 1D transforms (FastMultiplyLU::transform_1D, FastMultiplyLU.cpp:436-512):
 // for every element e and every entry of its output block,
 //   out[e][idx] = coef * sum_{s in N_t(e), L/U filter} sum_k in[s][idx, dim t <- k] * M[o_t(s)*n_from + k][o_t(e)*n_to + idx_t]
-// where N_t(e) is the vol or flx neighbour list of e in dimension t.  Instead
+// where N_t(e) is the vol or flx neighbour list of e in dimension t.  In two
+// and more dimensions these sums run planned (kernels_plan.cu); the sweep
+// kernels here serve one dimension and the explicitly chosen variants.  Instead
 // of one launch per transform, sweep j of every term of a range runs in one
 // launch (thread per term, element and output entry) with each term in its own
 // slice of the work buffer; the last sweep writes one slice per term and a
@@ -47,6 +49,8 @@ inline int ew_threads(int64_t n) {
     return t;
 }
 #define AMDG_EW_GRID(n) unsigned(((n) + ew_threads(n) - 1) / ew_threads(n)), ew_threads(n)
+// the same for launch_after: its kernels wait for the previous one before they touch memory
+#define AMDG_EW_AFTER(n) dim3(unsigned(((n) + ew_threads(n) - 1) / ew_threads(n))), unsigned(ew_threads(n)), 0, st
 
 // NODE_ROWS: the node is blockIdx.y and the thread's (element, entry) its index in the node's
 // E x out_block outputs (32-bit index arithmetic); else one 1D grid over all nodes' outputs
@@ -557,8 +561,9 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 // one thread per (element, point pair (q0, q1)): the four dofs of the pair, in the operation
 // order of HermInterpolation::eval_fp_Her_2D (Interplation.cpp:2045-2300) with f' = u, f'' = 1
 template <typename T>
-__global__ void herm_flux_burgers2d_kernel(const T* __restrict__ up, T* __restrict__ fp, int64_t n) {
+__global__ void herm_flux_burgers2d_kernel(const T* up, T* fp, int64_t n) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    wait_for_previous();
     if (i >= n) return;
     const int64_t e = i >> 2;
     const int q0 = int(i & 3) >> 1, q1 = int(i & 1);
@@ -577,8 +582,7 @@ template <typename T>
 cudaError_t launch_herm_flux_burgers2d(const T* up, T* fp, int64_t num_elements, cudaStream_t st) {
     const int64_t n = num_elements * 4;
     if (n == 0) return cudaSuccess;
-    herm_flux_burgers2d_kernel<T><<<AMDG_EW_GRID(n), 0, st>>>(up, fp, n);
-    return cudaGetLastError();
+    return launch_after(herm_flux_burgers2d_kernel<T>, AMDG_EW_AFTER(n), up, fp, n);
 }
 
 template cudaError_t launch_herm_flux_burgers2d<double>(const double*, double*, int64_t, cudaStream_t);
@@ -629,21 +633,26 @@ template cudaError_t launch_reduce_points_coef<double>(const double*, int, int64
 template cudaError_t launch_reduce_points_coef<float2>(const float2*, int, int64_t, int, int, const int32_t*,
                                                        const double*, double, double*, cudaStream_t);
 
-__global__ void to_df_kernel(const double* __restrict__ in, float2* __restrict__ out, int64_t n) {
+// the high parts by themselves (hi, unless null) are the FP32 state that the penalty reads
+__global__ void to_df_kernel(const double* in, float2* out, float* hi, int64_t n) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = from_double<float2>(in[i]);
+    wait_for_previous();
+    if (i >= n) return;
+    const float2 v = from_double<float2>(in[i]);
+    out[i] = v;
+    if (hi) hi[i] = v.x;
 }
 
-cudaError_t launch_to_df(const double* in, float2* out, int64_t n, cudaStream_t st) {
+cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    to_df_kernel<<<AMDG_EW_GRID(n), 0, st>>>(in, out, n);
-    return cudaGetLastError();
+    return launch_after(to_df_kernel, AMDG_EW_AFTER(n), in, out, hi, n);
 }
 
 // Eigen evaluates each vector expression elementwise with one rounding per operation (no contraction)
-__global__ void rk4_2nd_stage_kernel(int stage, double dt, const double* __restrict__ rhs, double* un, double* vn,
-                                     double* us, double* vs, double* su, double* sv, int64_t n) {
+__global__ void rk4_2nd_stage_kernel(int stage, double dt, const double* rhs, double* un, double* vn, double* us,
+                                     double* vs, double* su, double* sv, int64_t n) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    wait_for_previous();
     if (i >= n) return;
     if (stage < 0) {  // EulerODE2nd: u = u + dt v, v = v + dt rhs (ODESolver.cpp:409-414)
         const double u0 = un[i], v0 = vn[i];
@@ -675,8 +684,7 @@ __global__ void rk4_2nd_stage_kernel(int stage, double dt, const double* __restr
 cudaError_t launch_rk4_2nd_stage(int stage, double dt, const double* rhs, double* un, double* vn, double* us, double* vs,
                                  double* su, double* sv, int64_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    rk4_2nd_stage_kernel<<<AMDG_EW_GRID(n), 0, st>>>(stage, dt, rhs, un, vn, us, vs, su, sv, n);
-    return cudaGetLastError();
+    return launch_after(rk4_2nd_stage_kernel, AMDG_EW_AFTER(n), stage, dt, rhs, un, vn, us, vs, su, sv, n);
 }
 
 }  // namespace amdg

@@ -57,7 +57,7 @@ cudaError_t launch_reduce_points_coef(const Tin* buf, int count, int64_t E, int 
                                       const double* pts, double amp, double* out, cudaStream_t st);
 
 // double -> double-float (hi = float(v), lo = float(v - hi))
-cudaError_t launch_to_df(const double* in, float2* out, int64_t n, cudaStream_t st);
+cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, cudaStream_t st);
 
 // One RK4ODE2nd stage (ODESolver.cpp:579-615) given the right-hand side at (us, vs):
 // ku = dt vs, kv = dt rhs; stages 0-2 update (us, vs) from (un, vn) and the running sums

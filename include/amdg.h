@@ -249,7 +249,8 @@ amdg_status amdg_linear_destroy(amdg_linear_op* op);
  * algorithmic flops of one apply (2 * (k+1)^(dim+1) per pair). */
 amdg_status amdg_linear_stats(const amdg_linear_op* op, int64_t* pairs, double* flops_per_apply);
 /* Kernel variant per precision (variants[0] FP64, variants[1] mixed; 0 = one
- * thread per output coefficient, 1 = column variant, 2 = column variant whose
+ * thread per output coefficient, several threads per coefficient on small grids
+ * and k + 1 coefficients per thread on large FP32 ones, 1 = column variant, 2 = column variant whose
  * neighbour blocks arrive in shared memory by bulk asynchronous copies, mixed
  * only, 3 = the same bulk-copy ring with the per-dimension contraction
  * (FastMultiplyLU::transform_1D, FastMultiplyLU.cpp:436-512) on the tensor pipe
@@ -423,16 +424,18 @@ amdg_status amdg_burgers_rk3_steps(amdg_burgers_op* op, double dt, int nsteps, a
 enum { AMDG_LAGR_RHS_VOL = 0, AMDG_LAGR_RHS_FLX = 1, AMDG_LAGR_RHS_PENALTY = 2 };
 /* Algorithmic work of one right-hand side on the current element set (no reference counterpart):
  * the multiply-adds of every 1D transform sweep the right-hand side runs (2 flops each, from the
- * neighbour lists' L / full / U counts; terms whose first sweeps coincide share them) plus the
+ * neighbour lists' L / full / U counts, without the zero blocks that the planned transforms to point
+ * values leave out; sweeps that several terms share count once) plus the
  * surplus passes, and the (element, neighbour) pairs the sweeps visit.  Reads the lists back (synchronises): for measurement, not for the step loop. */
 amdg_status amdg_burgers_work(amdg_burgers_op* op, double* flops, double* transform_pairs);
-/* Kernel of the transform sweeps (no reference counterpart): 0 one thread per output entry; 1 one
- * thread per column of the transformed dimension, all its entries from one load of each input
- * value; 2 / 3 / 4 one warp per (term, element), its lanes over (column, neighbour phase), the
- * phases' partial sums added by shuffles, each warp serving 1 / 2 / 4 elements; -1 (default) 2 for
- * the FP32 sweeps of the mixed mode and 0 for the FP64 and double-float sweeps.  0 and 1 sum every
- * output in the same order (identical results); 2-4 sum in another fixed order (deterministic,
- * equal to rounding). */
+/* Kernel of the transform sweeps (no reference counterpart): -1 (default) planned sweeps, which add
+ * terms that end in the same transforms before these; the others run term by term: 0 one thread per
+ * output entry; 1 one thread per column of the transformed dimension, all its entries from one load
+ * of each input value; 2 / 3 / 4 one warp per (term, element), its lanes over (column, neighbour
+ * phase), the phases' partial sums added by shuffles, each warp serving 1 / 2 / 4 elements.  0 and 1
+ * sum every output in the same order (identical results); -1 and 2-4 sum in other fixed orders
+ * (deterministic, equal to rounding).  In one dimension -1 runs as 2 in the FP32 sweeps of the
+ * mixed mode and as 0 in the FP64 and double-float ones. */
 amdg_status amdg_burgers_set_sweep_variant(amdg_burgers_op* op, int variant);
 amdg_status amdg_lagr_interpolate(amdg_burgers_op* op, amdg_precision prec);
 amdg_status amdg_lagr_rhs_add(amdg_burgers_op* op, int group, const double* alpha, amdg_precision prec);
