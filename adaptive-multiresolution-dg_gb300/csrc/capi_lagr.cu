@@ -240,50 +240,37 @@ double wave_penalty_coef(const amdg_burgers_op* op) {
     return -op->sigma / (1.0 / std::pow(2.0, maxl));
 }
 
-// The nodes of every sweep tree on the device (grown when a tree is added; a step captured as a
-// graph refers to the buffer, so growing it drops the graph).
-amdg_status upload_nodes(amdg_burgers_op* op, cudaStream_t st) {
-    const size_t bytes = op->nodes.size() * sizeof(PartialSum);
-    if (bytes > op->nodes_cap) {
-        AMDG_CK(cudaStreamSynchronize(st));
-        cudaFree(op->d_nodes);
-        op->d_nodes = nullptr;
-        op->nodes_cap = 0;
-        const size_t want = 2 * bytes + 1024;
-        if (amdg::device_malloc(reinterpret_cast<void**>(&op->d_nodes), want) != cudaSuccess)
-            return fail(AMDG_ERR_NOMEM, "cudaMalloc failed (sweep trees)");
-        op->nodes_cap = want;
+// The device copy of a host list, grown when it no longer fits (a step captured as a graph refers to the
+// buffer, so growing it drops the graph).  The new buffer is allocated before the old one goes: a
+// failed allocation leaves the copy of the list as it was before the entries that did not fit.
+template <typename T>
+amdg_status upload_list(amdg_burgers_op* op, T** dst, size_t* cap, const std::vector<T>& host, cudaStream_t st) {
+    const size_t bytes = host.size() * sizeof(T);
+    if (bytes > *cap) {
+        const size_t want = bytes + bytes / 2 + 1024;
+        T* grown = nullptr;
+        if (amdg::device_malloc(&grown, want) != cudaSuccess) return fail(AMDG_ERR_NOMEM, "cudaMalloc failed (sweep lists)");
+        const cudaError_t e = cudaStreamSynchronize(st);
+        cudaFree(e == cudaSuccess ? *dst : grown);
+        AMDG_CK(e);
+        *dst = grown;
+        *cap = want;
         op->graph_version = -1;
     }
-    if (bytes) AMDG_CK(cudaMemcpyAsync(op->d_nodes, op->nodes.data(), bytes, cudaMemcpyHostToDevice, st));
-    AMDG_CK(cudaStreamSynchronize(st));  // op->nodes may change again before the copy would run
+    if (bytes) AMDG_CK(cudaMemcpyAsync(*dst, host.data(), bytes, cudaMemcpyHostToDevice, st));
+    AMDG_CK(cudaStreamSynchronize(st));  // the host list may change again before the copy would run
     return AMDG_OK;
+}
+
+// the nodes of every sweep tree on the device
+amdg_status upload_nodes(amdg_burgers_op* op, cudaStream_t st) {
+    return upload_list(op, &op->d_nodes, &op->nodes_cap, op->nodes, st);
 }
 
 // the nodes and products of the sweep plans on the device
 amdg_status upload_plans(amdg_burgers_op* op, cudaStream_t st) {
-    auto up = [&](auto** dst, size_t* cap, const auto& host) -> amdg_status {
-        const size_t bytes = host.size() * sizeof(host[0]);
-        if (bytes > *cap) {
-            AMDG_CK(cudaStreamSynchronize(st));
-            cudaFree(*dst);
-            *dst = nullptr;
-            *cap = 0;
-            const size_t want = 2 * bytes + 4096;
-            if (amdg::device_malloc(reinterpret_cast<void**>(dst), want) != cudaSuccess)
-                return fail(AMDG_ERR_NOMEM, "cudaMalloc failed (sweep plans)");
-            *cap = want;
-            op->graph_version = -1;  // a captured step read the old buffer
-        }
-        if (bytes) AMDG_CK(cudaMemcpyAsync(*dst, host.data(), bytes, cudaMemcpyHostToDevice, st));
-        return AMDG_OK;
-    };
-    amdg_status s;
-    if ((s = up(&op->d_plan_nodes, &op->plan_nodes_cap, op->plan_nodes)) != AMDG_OK ||
-        (s = up(&op->d_plan_products, &op->plan_products_cap, op->plan_products)) != AMDG_OK)
-        return s;
-    AMDG_CK(cudaStreamSynchronize(st));  // the host vectors may change again before the copies would run
-    return AMDG_OK;
+    if (amdg_status s = upload_list(op, &op->d_plan_nodes, &op->plan_nodes_cap, op->plan_nodes, st); s != AMDG_OK) return s;
+    return upload_list(op, &op->d_plan_products, &op->plan_products_cap, op->plan_products, st);
 }
 
 SweepPlan make_plan(amdg_burgers_op* op, int first, int count) {
@@ -316,9 +303,15 @@ amdg_status sweep_tree(amdg_burgers_op* op, int first, int count, SweepTree* out
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     AMDG_CK(cudaStreamIsCapturing(st, &cap));
     AMDG_REQUIRE(cap == cudaStreamCaptureStatusNone, AMDG_ERR_STATE, "sweep tree built during stream capture");
-    op->trees.push_back({{first, count}, build_sweep_tree(op->terms, first, count, op->grid->host.dim, &op->nodes)});
-    *out = op->trees.back().second;
-    return upload_nodes(op, st);
+    // the tree is kept only with its nodes on the device: a later call would launch without them
+    const size_t had = op->nodes.size();
+    *out = build_sweep_tree(op->terms, first, count, op->grid->host.dim, &op->nodes);
+    if (amdg_status s = upload_nodes(op, st); s != AMDG_OK) {
+        op->nodes.resize(had);
+        return s;
+    }
+    op->trees.push_back({{first, count}, *out});
+    return AMDG_OK;
 }
 
 // the sweep plan of the same terms
@@ -331,9 +324,15 @@ amdg_status sweep_plan(amdg_burgers_op* op, int first, int count, SweepPlan* out
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     AMDG_CK(cudaStreamIsCapturing(st, &cap));
     AMDG_REQUIRE(cap == cudaStreamCaptureStatusNone, AMDG_ERR_STATE, "sweep plan built during stream capture");
-    op->plans.push_back({{first, count}, make_plan(op, first, count)});
-    *out = op->plans.back().second;
-    return upload_plans(op, st);
+    const size_t had_nodes = op->plan_nodes.size(), had_products = op->plan_products.size();  // as sweep_tree
+    *out = make_plan(op, first, count);
+    if (amdg_status s = upload_plans(op, st); s != AMDG_OK) {
+        op->plan_nodes.resize(had_nodes);
+        op->plan_products.resize(had_products);
+        return s;
+    }
+    op->plans.push_back({{first, count}, *out});
+    return AMDG_OK;
 }
 
 // The default sweeps run planned (kernels_plan.cu); an explicit sweep variant runs term by term

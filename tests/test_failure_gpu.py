@@ -3,6 +3,7 @@ come back as AMDG_ERR_TIMEOUT with the state left as it was, and device allocati
 must come back as AMDG_ERR_NOMEM, with the library usable afterwards."""
 import numpy as np
 import pytest
+import torch
 
 import amdg
 import amdg_oracle as O
@@ -74,3 +75,56 @@ def test_device_allocation_failure_reports_nomem(ctx):
         g.close()
     finally:
         lib.amdg_debug_fail_device_allocations(-1)
+
+
+def _rhs(ctx, op, u):
+    du = torch.from_numpy(u.reshape(-1).copy()).cuda()
+    out = torch.zeros_like(du)
+    torch.cuda.synchronize()
+    op.rhs_device(du.data_ptr(), out.data_ptr())
+    ctx.synchronize()
+    return out.cpu().numpy()
+
+
+def test_sweep_lists_that_could_not_be_stored_are_stored_by_the_next_call(ctx):
+    """The sweep trees of a variant and the sweep plans of the term groups are built on first use.  With
+    no device memory left for them the call fails with AMDG_ERR_NOMEM, and a later call stores them:
+    the same results as of an operator that never failed."""
+    lib = amdg.load()
+    g = amdg.Grid(ctx, 3, 3, 2)
+    g.init_separable(O.wave_ic_terms(3))
+    u = g.coefficients()
+    op, fresh = amdg.WaveOperator(g, 10.0), amdg.WaveOperator(g, 10.0)
+    want = _rhs(ctx, fresh, u)
+    fresh.set_sweep_variant(0)
+    want0 = _rhs(ctx, fresh, u)
+
+    def by_groups():
+        g.set_rhs_zero()
+        for call, arg in ((op.interpolate, op.INTERP_GRADU), (op.rhs_add, op.RHS_FLX_GRADU), (op.rhs_add, op.RHS_VOL),
+                          (op.interpolate, op.INTERP_U), (op.rhs_add, op.RHS_FLX_U), (op.rhs_add, op.RHS_IPDG)):
+            call(arg)
+        ctx.synchronize()
+        return g.rhs().reshape(-1)
+
+    g.set_rhs_zero()
+    try:
+        lib.amdg_debug_fail_device_allocations(0)
+        with pytest.raises(amdg.AmdgError) as ei:
+            by_groups()
+        assert ei.value.status == NOMEM
+        lib.amdg_debug_fail_device_allocations(-1)
+        assert np.array_equal(by_groups(), want)
+        assert np.array_equal(_rhs(ctx, op, u), want)
+        op.set_sweep_variant(0)
+        lib.amdg_debug_fail_device_allocations(0)
+        with pytest.raises(amdg.AmdgError) as ei:
+            _rhs(ctx, op, u)
+        assert ei.value.status == NOMEM
+        lib.amdg_debug_fail_device_allocations(-1)
+        assert np.array_equal(_rhs(ctx, op, u), want0)
+    finally:
+        lib.amdg_debug_fail_device_allocations(-1)
+    op.close()
+    fresh.close()
+    g.close()
