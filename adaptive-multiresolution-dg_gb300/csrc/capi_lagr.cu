@@ -275,9 +275,25 @@ amdg_status upload_plans(amdg_burgers_op* op, cudaStream_t st) {
 
 SweepPlan make_plan(amdg_burgers_op* op, int first, int count) {
     const bool pv = first < op->n_pv_terms;
-    const int np = op->grid->host.k + 1;
-    return build_sweep_plan(op->terms, first, count, op->grid->host.dim, pv ? np : op->p1, pv ? op->p1 : np, np, pv,
-                            &op->plan_nodes, &op->plan_products);
+    const int np = op->grid->host.k + 1, dim = op->grid->host.dim;
+    const SweepPlan p = build_sweep_plan(op->terms, first, count, dim, pv ? np : op->p1, pv ? op->p1 : np, np, pv,
+                                         &op->plan_nodes, &op->plan_products);
+    for (int k = 0; !pv && k < p.count[dim - 1]; ++k)
+        op->plan_nodes[size_t(p.offset[dim - 1] + k)].long_mask = op->rhs_long_mask;
+    return p;
+}
+
+// the rules of the last sweeps that the whole operator shares (amdg_burgers_op)
+void set_plan_rules(amdg_burgers_op* op) {
+    const int np = op->grid->host.k + 1, dim = op->grid->host.dim, nterms = int(op->terms.size());
+    std::vector<PlanNode> nodes;
+    std::vector<PlanProduct> products;
+    const SweepPlan pv = build_sweep_plan(op->terms, 0, op->n_pv_terms, dim, np, op->p1, np, true, &nodes, &products);
+    op->pv_columns = plan_columns(pv.max_products, op->points);
+    const SweepPlan back = build_sweep_plan(op->terms, op->n_pv_terms, nterms - op->n_pv_terms, dim, op->p1, np, np, false,
+                                            &nodes, &products);
+    op->rhs_columns = plan_columns(back.max_products, op->grid->block);
+    for (int k = 0; k < back.count[dim - 1]; ++k) op->rhs_long_mask |= nodes[size_t(back.offset[dim - 1] + k)].long_mask;
 }
 
 // after a change of term coefficients: the nodes of every tree and plan again (the same structure:
@@ -467,6 +483,7 @@ amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count
     a.n_out = n_out;
     a.products = op->d_plan_products;
     a.max_products = plan.max_products;
+    a.columns = first < op->n_pv_terms ? op->pv_columns : op->rhs_columns;
     for (int i = 0; i < kNumLagrMats; ++i) a.mats[i] = m.m[i];
     a.rows = static_cast<const RowRec*>(op->d_rows);
     a.vol_nbr = reinterpret_cast<const int2*>(op->d_vol_nbr);
@@ -1122,6 +1139,7 @@ static amdg_status lagr_create(amdg_grid* g, int kind, const double* alpha, doub
     std::memcpy(op->weight, t.weight, sizeof(op->weight));
     transform_schedule(dim, &op->sched_dims, &op->sched_lu);
     build_terms(op);
+    set_plan_rules(op);
     amdg_status s;
     auto point_sines = [&]() -> amdg_status {
         if (amdg_status r = alloc_bytes(reinterpret_cast<void**>(&op->d_sines), t.pts.size() * sizeof(double)); r != AMDG_OK)

@@ -261,7 +261,7 @@ __device__ __forceinline__ void fibre_column(const Fibre<T>& f, int c, T (&acc)[
 }
 
 // whether element e's row along the node's non-"U" dimension (middle sweeps) or one of them (last
-// sweep) is long
+// sweep; of the transforms back, one of the operator's) is long
 template <typename T>
 __device__ __forceinline__ bool long_row(const PlanArgs<T>& a, const PlanNode& node, int64_t e) {
     for (int t = 0; t < a.dim; ++t)
@@ -526,6 +526,10 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
     }
 }
 
+bool plan_columns(int max_products, int out_block) {
+    return sizeof(float) * size_t(max_products) * size_t(out_block) <= kPartBytes;
+}
+
 bool plan_supported(int n_in, int n_out) {
     switch (n_in * 10 + n_out) {
         case 34: case 35: case 43: case 53: case 63: return true;
@@ -587,9 +591,8 @@ cudaError_t out_col(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
 template <typename T, int NF, int NT>
 cudaError_t out_nn(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
     if (shared_entries(a)) return out_col<T, NF, NT, false, kSharedPhases>(a, o, st);
-    // FP32: a thread per column where an element's parts fit
     if constexpr (std::is_same<T, float>::value)
-        if (sizeof(T) * size_t(a.max_products) * a.out_block <= kPartBytes) return out_col<T, NF, NT, true, 1>(a, o, st);
+        if (a.columns) return out_col<T, NF, NT, true, 1>(a, o, st);
     return out_col<T, NF, NT, false, 1>(a, o, st);
 }
 

@@ -51,6 +51,7 @@ struct PlanArgs {
     const PlanNode* nodes;           // nodes of this sweep, node = blockIdx.y
     const PlanProduct* products;
     int num_nodes, max_products;     // products of the largest node
+    bool columns;                    // last sweep, FP32: a thread per column (plan_columns)
     int out_block;                   // output entries per element
     bool first_sweep;                // products read src[in], else in + in * in_slice
     const T* mats[kNumLagrMats];     // blocked by order pair
@@ -80,6 +81,10 @@ template <typename T>
 cudaError_t launch_plan_sweep(const PlanArgs<T>& a, cudaStream_t st);
 template <typename T>
 cudaError_t launch_plan_out(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st);
+// whether the FP32 last sweep of nodes of up to max_products products takes a thread per column: where an
+// element's parts fit the shared memory.  The two forms add the neighbours in different orders, so an
+// operator decides once, from all its terms, and its term groups by themselves follow that.
+bool plan_columns(int max_products, int out_block);
 // whether the (n_in, n_out) pair has kernels
 bool plan_supported(int n_in, int n_out);
 
