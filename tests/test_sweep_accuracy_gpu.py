@@ -1,0 +1,106 @@
+"""Accuracy of the planned transform sweeps on random coefficients: element by element, where a wrong or
+missing neighbour of one element shows, and on average against the sweeps term by term."""
+import numpy as np
+import pytest
+import torch
+
+import amdg
+import amdg_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def make(ctx, kind, dim, nmax, shape):
+    if shape == "adaptive":
+        g = amdg.Grid(ctx, dim, nmax, 2, level_init=3)
+        g.init_separable_adaptive(O.wave_ic_terms(dim) if kind == "wave" else O.burgers_ic_terms(dim), 2e-6)
+    else:
+        g = amdg.Grid(ctx, dim, nmax, 2, sparse=shape == "sparse")
+    op = amdg.WaveOperator(g, 10.0) if kind == "wave" else amdg.BurgersOperator(g, 0.825, hermite=kind == "hermite")
+    return g, op
+
+
+def randomise(g, seed, decay):
+    """Normal coefficients, an element's scaled by 2^(-decay times its level sum)."""
+    levels, _ = g.elements()
+    scale = 2.0 ** (-decay * np.asarray(levels).reshape(g.num_elements, -1).sum(1))
+    u = np.random.default_rng(seed).standard_normal((g.num_elements, g.block)) * scale[:, None]
+    g.set_coefficients(u)
+    return u
+
+
+def rhs(ctx, g, op, prec):
+    du = torch.from_numpy(g.coefficients().reshape(-1).copy()).cuda()
+    out = torch.zeros_like(du)
+    torch.cuda.synchronize()
+    op.rhs_device(du.data_ptr(), out.data_ptr(), prec)
+    ctx.synchronize()
+    return out.cpu().numpy().reshape(g.num_elements, g.block)
+
+
+def per_element(err, ref):
+    return (np.linalg.norm(err, axis=1) / np.linalg.norm(ref, axis=1)).max()
+
+
+# both sides of the size up to which lanes share an entry, rows to share out, FP32 columns with one and
+# several dimensions in a node, odd lengths of rows, blocks in windows
+SHAPES = [("burgers", 3, 4, "sparse"), ("burgers", 3, 7, "sparse"), ("burgers", 2, 8, "sparse"),
+          ("burgers", 3, 7, "adaptive"), ("burgers", 4, 5, "sparse"), ("burgers", 5, 4, "sparse"),
+          ("burgers", 6, 3, "sparse"), ("hermite", 2, 6, "sparse"), ("hermite", 2, 8, "sparse"),
+          ("wave", 2, 5, "full"), ("wave", 2, 7, "full"), ("wave", 3, 5, "sparse"), ("wave", 4, 4, "sparse")]
+
+
+@pytest.mark.parametrize("kind,dim,nmax,shape", SHAPES)
+def test_mixed_right_hand_side_element_by_element(ctx, kind, dim, nmax, shape):
+    """The largest relative error of an element's block against FP64 stays within four times that of the
+    sweeps term by term (FP32 roundings of the same sums in another order); a neighbour left out or a
+    wrong block would make it some 1e-2."""
+    g, op = make(ctx, kind, dim, nmax, shape)
+    randomise(g, 3, 1.0)
+    errs = []
+    for variant in (-1, 0):
+        op.set_sweep_variant(variant)
+        exact = rhs(ctx, g, op, amdg.FP64)
+        errs.append(per_element(rhs(ctx, g, op, amdg.MIXED) - exact, exact))
+    assert errs[0] <= 4.0 * errs[1], errs
+    op.close()
+    g.close()
+
+
+@pytest.mark.parametrize("kind,dim,nmax", [("burgers", 2, 7), ("burgers", 3, 5), ("burgers", 4, 3), ("wave", 2, 6)])
+def test_right_hand_side_element_by_element_against_the_oracle(ctx, kind, dim, nmax):
+    """FP64: every element's block to 1e-10 of its norm (a block is up to some 1e2 smaller than the terms
+    that it is the sum of; the terms agree to the 1e-12 of the whole field)."""
+    g, op = make(ctx, kind, dim, nmax, "sparse")
+    u = randomise(g, 4, 1.0)
+    levels, support = g.elements()
+    if kind == "wave":
+        ref = O.wave_rhs(dim, nmax, 2, levels, support, u, 10.0)
+    else:
+        ref = O.burgers_rhs(dim, nmax, 2, levels, support, u, 0.825)[0]
+    ref = np.asarray(ref).reshape(g.num_elements, g.block)
+    assert per_element(rhs(ctx, g, op, amdg.FP64) - ref, ref) <= 1e-10
+    op.close()
+    g.close()
+
+
+@pytest.mark.parametrize("kind,dim,nmax,shape", [("hermite", 2, 6, "sparse"), ("hermite", 2, 7, "adaptive"),
+                                                 ("burgers", 2, 5, "sparse"), ("burgers", 3, 5, "sparse"),
+                                                 ("wave", 2, 4, "full"), ("wave", 2, 5, "sparse")])
+def test_mixed_error_is_no_larger_than_term_by_term(ctx, kind, dim, nmax, shape):
+    """The L2 error of the mixed right-hand side against FP64, geometric mean over 40 states with the
+    coefficients of a smooth function (2^-3 per level): no larger than that of the sweeps term by term
+    with a warp per element."""
+    g, op = make(ctx, kind, dim, nmax, shape)
+    logs = []
+    for seed in range(40):
+        randomise(g, seed, 3.0)
+        errs = []
+        for variant in (-1, 2):
+            op.set_sweep_variant(variant)
+            exact = rhs(ctx, g, op, amdg.FP64)
+            errs.append(np.linalg.norm(rhs(ctx, g, op, amdg.MIXED) - exact))
+        logs.append(np.log(errs[0] / errs[1]))
+    assert np.exp(np.mean(logs)) <= 1.0
+    op.close()
+    g.close()
