@@ -508,7 +508,7 @@ struct amdg_burgers_op {
     // wave: element set and arithmetic of the K grad u [0] and K u [1] interpolations amdg_wave_interpolate kept
     int64_t wave_interp_version[2] = {-1, -1};
     int wave_interp_prec[2] = {-1, -1};
-    int chunk = 1;  // terms per launch
+    int chunk = 1;  // terms per launch sequence (terms_per_launch of the element set)
     int sweep_variant = -1;  // transform sweep kernel: -1 the planned sweeps, else one sweep per term: 0 thread per output entry, 1 thread per
                              // column, 2 / 3 / 4 warp per (node, element) with 1 / 2 / 4 elements per warp
     // work buffers sized for FP64: E x p1^dim doubles each, the sweep buffers and

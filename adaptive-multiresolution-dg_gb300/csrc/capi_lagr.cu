@@ -355,6 +355,21 @@ amdg_status sweep_plan(amdg_burgers_op* op, int first, int count, SweepPlan* out
 // through the sweep trees, and so does one dimension, where every term is a single sweep.
 bool planned(const amdg_burgers_op* op) { return op->sweep_variant < 0 && op->grid->host.dim > 1; }
 
+// Terms that one launch sequence may evaluate on E elements: all of them unless their three slices per
+// term (two sweep buffers and the output; buffers have room for half as many elements again) would
+// pass kTermBudget bytes.  A function of the element count alone, not of the buffers an earlier and
+// larger element set left behind: the ranges decide which terms are added before their transforms.
+int64_t room_for(int64_t E) { return E + E / 2 + 16; }
+int terms_per_launch(const amdg_burgers_op* op, int64_t E) {
+    const int64_t slices = 3 * room_for(E) * op->points * int64_t(sizeof(double));
+    return int(std::max<int64_t>(1, std::min<int64_t>(int64_t(op->terms.size()), int64_t(kTermBudget) / slices)));
+}
+// bytes of one sweep buffer with room for `cap` elements: terms_per_launch(E) slices of any E <= cap
+size_t slices_bytes(const amdg_burgers_op* op, int64_t cap) {
+    const size_t one = size_t(cap) * op->points * sizeof(double);
+    return std::max(one, std::min(op->terms.size() * one, 2 * kTermBudget / 9));
+}
+
 // The terms [first, first + total) in the ranges that one launch sequence evaluates: all of them, or,
 // past the term budget, pieces of at most `chunk` terms of one group each, so that a group's sums do
 // not depend on what is evaluated beside it.
@@ -998,7 +1013,7 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
     }
     const int64_t E = g->host.num_elements;
     if (E > op->capacity) {
-        const int64_t cap = E + E / 2 + 16;
+        const int64_t cap = room_for(E);
         void* bufs[] = {op->w_up, op->w_fu, op->w_a, op->w_b, op->w_u, op->w_s0, op->w_s1, op->w_slots,
                         op->d_u1, op->d_u2, op->d_rhs64, op->d_pred, op->w_fields, op->d_v1, op->d_su, op->d_sv};
         for (void* p : bufs) cudaFree(p);
@@ -1007,11 +1022,7 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
         op->capacity = 0;
         const size_t work = size_t(cap) * op->points * sizeof(double);
         const size_t vec = size_t(cap) * g->block * sizeof(double);
-        // terms per launch: all of them unless their three slices per term
-        // (two sweep buffers and the output) would pass kTermBudget bytes
-        const int nterms = int(op->terms.size());
-        op->chunk = int(std::max<int64_t>(1, std::min<int64_t>(nterms, int64_t(kTermBudget / (3 * work)))));
-        const size_t slices = size_t(op->chunk) * work;
+        const size_t slices = slices_bytes(op, cap);
         if ((s = alloc_bytes(&op->w_up, work)) != AMDG_OK || (s = alloc_bytes(&op->w_fu, work)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_a, work)) != AMDG_OK || (s = alloc_bytes(&op->w_b, work)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_u, vec + vec / 2)) != AMDG_OK || (s = alloc_bytes(&op->w_s0, slices)) != AMDG_OK ||
@@ -1029,6 +1040,7 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
             return s;
         op->capacity = cap;
     }
+    op->chunk = terms_per_launch(op, E);
     if (op->kind == 1) {  // the IPDG coefficient follows the finest level
         const double c = wave_penalty_coef(op);
         bool changed = false;

@@ -15,7 +15,9 @@
 //
 // In both, the outputs of elements with a row of more than kLongRow neighbours are left out of that
 // mapping and dealt to the CTAs as extra units, one unit to a CTA before its own work: kLongPhases
-// threads per output entry, each a fixed subset of the neighbours, their sums added in a fixed order.  Every sum's order depends on the element set alone.
+// threads per output entry, each a fixed subset of the neighbours, their sums added in a fixed order.  Every
+// sum's order depends on the operator and the element set alone (the plan's term range follows the element
+// count).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -104,3 +104,44 @@ def test_mixed_error_is_no_larger_than_term_by_term(ctx, kind, dim, nmax, shape)
     assert np.exp(np.mean(logs)) <= 1.0
     op.close()
     g.close()
+
+
+# grids on which not all terms fit one launch sequence: the fields of the wave one by one and its groups in
+# pieces; four and eight pieces of the transforms to point values, groups term by term
+PIECES = [("wave", 3, 5), ("burgers", 4, 4), ("burgers", 5, 3)]
+
+
+@pytest.mark.parametrize("kind,dim,nmax", PIECES)
+def test_terms_in_pieces_element_by_element(ctx, kind, dim, nmax):
+    """FP64 against the sweeps term by term to 1e-10 of an element's norm, mixed as above."""
+    g, op = make(ctx, kind, dim, nmax, "full")
+    randomise(g, 5, 1.0)
+    exact, errs = [], []
+    for variant in (-1, 0):
+        op.set_sweep_variant(variant)
+        exact.append(rhs(ctx, g, op, amdg.FP64))
+        errs.append(per_element(rhs(ctx, g, op, amdg.MIXED) - exact[-1], exact[-1]))
+    assert per_element(exact[0] - exact[1], exact[1]) <= 1e-10
+    assert errs[0] <= 4.0 * errs[1], errs
+    op.close()
+    g.close()
+
+
+@pytest.mark.parametrize("prec", [amdg.FP64, amdg.MIXED])
+def test_sums_do_not_depend_on_an_earlier_larger_grid(ctx, prec):
+    """A wave operator whose grid shrank from 32,768 elements, where its groups go in pieces, to the
+    coarse levels: the same bits as of a new operator on that grid."""
+    g, op = make(ctx, "wave", 3, 5, "full")
+    levels, _ = g.elements()
+    keep = np.asarray(levels).reshape(g.num_elements, -1).sum(1) <= 6
+    u = np.random.default_rng(6).standard_normal((g.num_elements, g.block)) * keep[:, None]
+    g.set_coefficients(u)
+    rhs(ctx, g, op, prec)
+    g.coarsen(1e-6)
+    assert g.num_elements == keep.sum()
+    got = rhs(ctx, g, op, prec)
+    new = amdg.WaveOperator(g, 10.0)
+    assert np.array_equal(got, rhs(ctx, g, new, prec))
+    new.close()
+    op.close()
+    g.close()
