@@ -499,6 +499,11 @@ struct amdg_burgers_op {
     // the transforms to points and back, and the dimensions whose long rows the transforms back share out
     bool pv_columns = false, rhs_columns = false;
     int32_t rhs_long_mask = 0;
+    // per sweep of the transforms to point values: the last evaluation (they are numbered) with an input
+    // that was not finite.  (A step replayed as a graph keeps its numbers: after such an evaluation it
+    // takes the whole lists until it is captured again.)
+    uint32_t* d_nonfinite = nullptr;
+    uint32_t evaluation = 0;
     void* d_rows = nullptr;          // amdg::RowRec per (element, dimension)
     int32_t* d_long = nullptr;       // long rows: counts per dimension (kMaxDim), then the elements per dimension
     int64_t long_stride = 0;

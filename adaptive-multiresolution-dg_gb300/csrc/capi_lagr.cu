@@ -480,6 +480,18 @@ amdg_status run_terms(amdg_burgers_op* op, const Mats<T>& m, int first, int coun
     return AMDG_OK;
 }
 
+// the mark of the inputs of sweep j of the transforms to point values, in the current evaluation
+NonfiniteMark input_mark(const amdg_burgers_op* op, int j) { return NonfiniteMark{op->d_nonfinite + j, op->evaluation}; }
+
+// begins an evaluation of point values of the FP64 state u
+amdg_status begin_evaluation(amdg_burgers_op* op, const double* u, cudaStream_t st) {
+    ++op->evaluation;
+    if (!planned(op)) return AMDG_OK;
+    AMDG_CK(launch_find_nonfinite(u, op->grid->dof, input_mark(op, 0), st));
+    op->grid->ctx->launches++;
+    return AMDG_OK;
+}
+
 // The planned sweeps of terms [first, first + count), the last one ending in `o`.
 template <typename T>
 amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count, int n_in, int n_out,
@@ -508,9 +520,13 @@ amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count
     a.long_count = op->d_long;
     a.long_rows = op->d_long + kMaxDim;
     a.long_stride = op->long_stride;
+    const bool pv = first < op->n_pv_terms;
     const T* cur = nullptr;
     for (int j = 0; j < dim; ++j) {
         a.first_sweep = j == 0;
+        // (nothing has looked through the FP32 state of amdg_burgers_point_values and _flux_coefficients)
+        a.in_mark = pv && (j > 0 || !std::is_same<T, float>::value) ? input_mark(op, j) : NonfiniteMark{};
+        a.out_mark = pv && j + 1 < dim ? input_mark(op, j + 1) : NonfiniteMark{};
         a.in = cur;
         a.in_slice = j == 0 ? 0 : E * ipow(n_out, j) * ipow(n_in, dim - j);
         a.out_block = ipow(n_out, j + 1) * ipow(n_in, dim - j - 1);
@@ -538,6 +554,11 @@ amdg_status eval_point_values(amdg_burgers_op* op, const Mats<T>& m, const T* u,
     const bool herm = op->kind == 3;  // the Hermite flux needs the slopes too: applied after the sum
     T* slots = static_cast<T*>(op->w_slots);
     const T* src[1] = {u};
+    if constexpr (std::is_same<T, double>::value) {
+        if (amdg_status r = begin_evaluation(op, u, st); r != AMDG_OK) return r;
+    } else {
+        ++op->evaluation;
+    }
     if (planned(op)) {
         const auto ranges = term_ranges(op, 0, op->n_pv_terms);
         for (size_t i = 0; i < ranges.size(); ++i) {
@@ -573,7 +594,8 @@ amdg_status eval_point_values_df(amdg_burgers_op* op, const double* u, double* u
     const int np = op->grid->host.k + 1;
     const int64_t n = op->grid->host.num_elements * op->points;
     float2* udf = static_cast<float2*>(op->w_u);
-    AMDG_CK(launch_to_df(u, udf, u32, op->grid->dof, st));
+    ++op->evaluation;
+    AMDG_CK(launch_to_df(u, udf, u32, op->grid->dof, input_mark(op, 0), st));
     op->grid->ctx->launches++;
     float2* slots = static_cast<float2*>(op->w_slots);
     const float2* src[1] = {udf};
@@ -718,10 +740,12 @@ amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, c
     Tp* slots = static_cast<Tp*>(op->w_slots);
     const Tp* src[1];
     if constexpr (df) {
-        AMDG_CK(launch_to_df(u, static_cast<float2*>(op->w_u), u32, g->dof, st));
+        ++op->evaluation;
+        AMDG_CK(launch_to_df(u, static_cast<float2*>(op->w_u), u32, g->dof, input_mark(op, 0), st));
         op->grid->ctx->launches++;
         src[0] = static_cast<const float2*>(op->w_u);
     } else {
+        if (amdg_status r = begin_evaluation(op, u, st); r != AMDG_OK) return r;
         src[0] = u;
     }
     const Mats<Tp> m = [&] {
@@ -1170,6 +1194,7 @@ static amdg_status lagr_create(amdg_grid* g, int kind, const double* alpha, doub
         (s = upload_df(&op->df_a2p, t.a2p)) != AMDG_OK || (kind == 1 && (s = upload_df(&op->df_a2pd, t.a2pd)) != AMDG_OK) ||
         (s = upload_vec(&op->d_anc_point, t.anc_point)) != AMDG_OK || (s = upload_vec(&op->d_anc_rank, t.anc_rank)) != AMDG_OK ||
         (s = upload_vec(&op->d_terms, op->terms)) != AMDG_OK || (s = upload_vec(&op->d_seen, op->seen)) != AMDG_OK ||
+        (s = upload_vec(&op->d_nonfinite, std::vector<uint32_t>(kMaxDim, 0u))) != AMDG_OK ||
         (s = burgers_sync(op)) != AMDG_OK) {
         amdg_burgers_destroy(op);
         return s;
@@ -1204,7 +1229,7 @@ amdg_status amdg_burgers_destroy(amdg_burgers_op* op) {
                     op->d_feat, op->d_prob, op->d_a2pd, op->d_ljv, op->d_pts, op->f_a2pd, op->f_ljv,
                     op->w_fields, op->d_v1, op->d_su, op->d_sv, op->df_a2p, op->df_a2pd,
                     op->d_anc_order, op->d_topo_cnt, op->d_cls, op->d_nodes, op->d_plan_nodes, op->d_plan_products,
-                    op->d_rows, op->d_long, op->d_sines, op->d_seen};
+                    op->d_rows, op->d_long, op->d_sines, op->d_seen, op->d_nonfinite};
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(op->h_cls);
     delete op;

@@ -56,8 +56,27 @@ template <typename Tin>
 cudaError_t launch_reduce_points_coef(const Tin* buf, int count, int64_t E, int dim, int p1, const int32_t* order,
                                       const double* pts, double amp, double* out, cudaStream_t st);
 
+// Where a kernel notes that a value it wrote is not finite: *at = the number of the evaluation that
+// reads the value (nullptr: not noted).  The transforms to point values read it (inputs_finite in
+// kernels_plan.cu).
+struct NonfiniteMark {
+    uint32_t* at;
+    uint32_t evaluation;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ bool finite_bits(double v) { return (uint32_t(__double2hiint(v)) & 0x7ff00000u) != 0x7ff00000u; }
+__device__ __forceinline__ bool finite_bits(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool finite_bits(float2 v) { return finite_bits(v.x); }
+template <typename T>
+__device__ __forceinline__ void note(const NonfiniteMark& m, T v) {
+    if (m.at && !finite_bits(v)) *m.at = m.evaluation;
+}
+#endif
+// note(mark, u[i]) for n entries
+cudaError_t launch_find_nonfinite(const double* u, int64_t n, NonfiniteMark mark, cudaStream_t st);
+
 // double -> double-float (hi = float(v), lo = float(v - hi))
-cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, cudaStream_t st);
+cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, NonfiniteMark mark, cudaStream_t st);
 
 // One RK4ODE2nd stage (ODESolver.cpp:579-615) given the right-hand side at (us, vs):
 // ku = dt vs, kv = dt rhs; stages 0-2 update (us, vs) from (un, vn) and the running sums

@@ -16,7 +16,8 @@ namespace amdg {
 // flx neighbours), and how many of the finer vol neighbours, at the end of the list, hold none of the
 // element's interpolation points.  Two 16-byte loads give a thread all of it at once.
 //
-// Those last neighbours have a zero block in the transforms to point values, which stop before them: a
+// Those last neighbours have a zero block in the transforms to point values, which stop before them
+// where every input of the sweep is finite: a
 // point lies in one neighbour of each finer level, while the element meets 2^m of them m levels
 // down.  They are a quarter to a third of all neighbours and most of a long row's (mixed wave step on
 // 16,384 elements in 2D 2212 -> 2063 us, mixed 3D step on 4,096 1266 -> 1185 us).
@@ -65,6 +66,7 @@ struct PlanArgs {
     const int32_t* long_count;       // [dim] long rows of each dimension
     const int32_t* long_rows;        // [dim][long_stride] their elements
     int64_t long_stride;
+    NonfiniteMark in_mark, out_mark; // transforms to point values: of the sweep's inputs, of its outputs
 };
 
 struct PlanOut {
