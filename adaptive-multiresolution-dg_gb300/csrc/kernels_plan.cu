@@ -112,7 +112,7 @@ __device__ __forceinline__ Fibre<T> fibre_of(const PlanArgs<T>& a, const PlanPro
 // neighbours its error bound, 36 units of 2^-48, is below that of six double-float multiplications and
 // additions (about 60), for 12 instructions a product instead of 27.
 __device__ __forceinline__ float2 df_product(float2 x, float2 m) {
-    const float p = x.x * m.x;
+    const float p = __fmul_rn(x.x, m.x);
     return make_float2(p, fmaf(x.x, m.y, fmaf(x.y, m.x, fmaf(x.x, m.x, -p))));
 }
 __device__ __forceinline__ float2 df_dot(float2 s, float2 x, float2 m) {
@@ -127,7 +127,7 @@ __device__ __forceinline__ float2 exact_dot(const float (&x)[NF], const float (&
     float s[NF], lost = 0.0f;
 #pragma unroll
     for (int k = 0; k < NF; ++k) {
-        s[k] = x[k] * m[k];
+        s[k] = __fmul_rn(x[k], m[k]);
         lost += fmaf(x[k], m[k], -s[k]);
     }
 #pragma unroll

@@ -10,7 +10,8 @@ namespace amdg {
 // ---- double-float arithmetic (float2 = hi + lo, |lo| <= ulp(hi)/2, about 48 bits) -------------
 // The error-free transformations two-sum (Knuth) and the FMA-based exact product, combined as in
 // the double-double algorithms of Hida, Li and Bailey ("accurate" addition): the point-value
-// sweeps of the mixed mode run on the FP32 pipe with near-FP64 accuracy.
+// sweeps of the mixed mode run on the FP32 pipe with near-FP64 accuracy.  Products whose rounding is taken
+// apart are __fmul_rn: the compiler must not contract them into the additions that follow.
 __device__ __forceinline__ float2 df_two_sum(float a, float b) {
     const float s = a + b;
     const float bb = s - a;
@@ -29,7 +30,7 @@ __device__ __forceinline__ float2 df_add(float2 a, float2 b) {
     return df_quick_two_sum(s.x, s.y);
 }
 __device__ __forceinline__ float2 df_mul(float2 a, float2 b) {
-    const float p = a.x * b.x;
+    const float p = __fmul_rn(a.x, b.x);
     float e = fmaf(a.x, b.x, -p);
     e = fmaf(a.x, b.y, e);
     e = fmaf(a.y, b.x, e);
