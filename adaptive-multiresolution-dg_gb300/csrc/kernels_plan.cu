@@ -619,13 +619,6 @@ bool plan_columns(int max_products, int out_block) {
     return sizeof(float) * size_t(max_products) * size_t(out_block) <= kPartBytes;
 }
 
-bool plan_supported(int n_in, int n_out) {
-    switch (n_in * 10 + n_out) {
-        case 34: case 35: case 43: case 53: case 63: return true;
-        default: return false;
-    }
-}
-
 namespace {
 
 // lanes per output entry: on grids of few outputs a launch lasts as long as one thread's chain over its
@@ -687,15 +680,19 @@ cudaError_t out_nn(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st) {
 
 }  // namespace
 
-#define AMDG_PLAN_CASES(F)                                   \
-    switch (a.n_in * 10 + a.n_out) {                         \
-        case 34: return F<T, 3, 4>;                          \
-        case 35: return F<T, 3, 5>;                          \
-        case 43: return F<T, 4, 3>;                          \
-        case 53: return F<T, 5, 3>;                          \
-        case 63: return F<T, 6, 3>;                          \
-        default: return nullptr;                             \
-    }
+// The pairs of entries per dimension that occur: points of degree 3 (or cubic Hermite) and, for the wave, 4
+// from Alpert coefficients and back, also from points of degree 5 in FP64 (initialisation); double-float to
+// points only.
+#define AMDG_PLAN_CASES(F)                                                                      \
+    constexpr bool df = std::is_same<T, float2>::value, f32 = std::is_same<T, float>::value;    \
+    switch (a.n_in * 10 + a.n_out) {                                                            \
+        case 34: return F<T, 3, 4>;                                                             \
+        case 35: if constexpr (!f32) return F<T, 3, 5>; break;                                  \
+        case 43: if constexpr (!df) return F<T, 4, 3>; break;                                   \
+        case 53: if constexpr (!df) return F<T, 5, 3>; break;                                   \
+        case 63: if constexpr (!df && !f32) return F<T, 6, 3>; break;                           \
+    }                                                                                           \
+    return nullptr;
 
 template <typename T>
 static cudaError_t (*pick_sweep(const PlanArgs<T>& a))(const PlanArgs<T>&, cudaStream_t) { AMDG_PLAN_CASES(sweep_nn) }

@@ -87,8 +87,6 @@ cudaError_t launch_plan_out(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t
 // element's parts fit the shared memory.  The two forms add the neighbours in different orders, so an
 // operator decides once, from all its terms, and its term groups by themselves follow that.
 bool plan_columns(int max_products, int out_block);
-// whether the (n_in, n_out) pair has kernels
-bool plan_supported(int n_in, int n_out);
 
 // row records of host-built neighbour lists (vol_skip: finer vol neighbours without a point), long rows
 // appended to long_rows (long_count zeroed before)
