@@ -1050,7 +1050,7 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
         if ((s = alloc_bytes(&op->w_up, work)) != AMDG_OK || (s = alloc_bytes(&op->w_fu, work)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_a, work)) != AMDG_OK || (s = alloc_bytes(&op->w_b, work)) != AMDG_OK ||
             (s = alloc_bytes(&op->w_u, vec + vec / 2)) != AMDG_OK || (s = alloc_bytes(&op->w_s0, slices)) != AMDG_OK ||
-            (s = alloc_bytes(&op->w_s1, slices)) != AMDG_OK || (s = alloc_bytes(&op->w_slots, slices)) != AMDG_OK ||
+            (s = alloc_bytes(&op->w_s1, slices)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_u1), vec)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_u2), vec)) != AMDG_OK ||
             (s = alloc_bytes(reinterpret_cast<void**>(&op->d_rhs64), vec)) != AMDG_OK ||
@@ -1064,6 +1064,8 @@ amdg_status burgers_sync(amdg_burgers_op* op) {
             return s;
         op->capacity = cap;
     }
+    // the terms' slices: only the sweeps term by term write them
+    if (!planned(op) && !op->w_slots && (s = alloc_bytes(&op->w_slots, slices_bytes(op, op->capacity))) != AMDG_OK) return s;
     op->chunk = terms_per_launch(op, E);
     if (op->kind == 1) {  // the IPDG coefficient follows the finest level
         const double c = wave_penalty_coef(op);

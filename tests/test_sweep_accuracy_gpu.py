@@ -145,3 +145,20 @@ def test_sums_do_not_depend_on_an_earlier_larger_grid(ctx, prec):
     new.close()
     op.close()
     g.close()
+
+
+def test_slices_of_the_terms_are_allocated_for_the_sweeps_term_by_term_only(ctx):
+    """The planned sweeps write no slice per term: their operator holds that memory only after a variant
+    that does was chosen (32,768 elements x 64 points, some 20 terms: hundreds of MB)."""
+    g = amdg.Grid(ctx, 3, 5, 2, sparse=False)
+    op = amdg.BurgersOperator(g, 0.825)
+    randomise(g, 8, 1.0)
+    exact = rhs(ctx, g, op, amdg.FP64)
+    free = torch.cuda.mem_get_info()[0]
+    assert np.array_equal(rhs(ctx, g, op, amdg.FP64), exact)
+    assert free - torch.cuda.mem_get_info()[0] < 64 << 20
+    op.set_sweep_variant(0)
+    rhs(ctx, g, op, amdg.FP64)
+    assert free - torch.cuda.mem_get_info()[0] > 128 << 20
+    op.close()
+    g.close()
