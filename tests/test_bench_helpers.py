@@ -73,3 +73,21 @@ def test_refine_labels_are_the_criterion():
     norms = np.sqrt(np.sum(g.u ** 2, axis=1))
     assert np.array_equal(lab, np.where(norms > 1e-3, 0, 1))
     assert set(lab.tolist()) == {0, 1}
+
+
+def test_printed_line_is_short_and_keeps_the_headline():
+    """All of the headline's entries unchanged, the rates of the other workloads, in a few KB."""
+    import json
+
+    arm = {"value": 1.5, "wall_s": 2.0, "host_phase_ms": {"rhs": 1.0}, "note": "x" * 400}
+    line = {k: {"k": k} for k in bench.HEADLINE_KEYS}
+    line.update(value=3.25, metric="m", linear6d=dict(arm, cpu_baseline={"value": 7.0}, unit="u"),
+                wave2d_adaptive={"workload": "y" * 500, "arms": {f"arm{i}": dict(arm) for i in range(20)}},
+                linear4d={"fp64": dict(arm), "mixed": dict(arm)}, notes=["z"] * 100)
+    short = bench.headline(json.loads(json.dumps(line)))
+    assert all(short[k] == line[k] for k in bench.HEADLINE_KEYS)
+    others = short["other_workloads_value"]
+    assert others["linear6d"] == {"value": 1.5, "cpu_baseline": 7.0}
+    assert others["linear4d"] == {"fp64": 1.5, "mixed": 1.5}
+    assert others["wave2d_adaptive"]["arms"]["arm19"] == 1.5
+    assert len(json.dumps(line)) > 10000 and len(json.dumps(short)) < 4000
