@@ -1068,6 +1068,9 @@ amdg_status grid_device_refine(amdg_grid* g, double eps, const uint8_t* d_force,
     cudaStream_t st = stream_of(g);
     AdaptStats* dst = static_cast<AdaptStats*>(d.stats);
     AMDG_CK(cudaMemsetAsync(dst, 0, kStatsReset, st));
+    // the marks put the added keys into the hash: it no longer holds the element set alone, and a call that
+    // fails below must not leave it for the next one, which would take those keys for already marked
+    d.hash_version = -1;
     if (E > 0) {
         int width = 2;  // lanes per element: 12 -> 6 us at 2,104 elements in three dimensions
         while (width < 2 * ks.dim) width *= 2;
@@ -1087,7 +1090,10 @@ amdg_status grid_device_refine(amdg_grid* g, double eps, const uint8_t* d_force,
     }
     const int64_t n_new = hs.count;
     if (added) *added = n_new;
-    if (n_new == 0) return AMDG_OK;
+    if (n_new == 0) {
+        d.hash_version = g->version;
+        return AMDG_OK;
+    }
     const int64_t En = E + n_new;
     if (En > (int64_t(1) << 31) - 1) return fail(AMDG_ERR_CAPACITY, "more than 2^31-1 elements");
     // every allocation before the first change, so a failure leaves the element set as it was

@@ -128,3 +128,36 @@ def test_sweep_lists_that_could_not_be_stored_are_stored_by_the_next_call(ctx):
     op.close()
     fresh.close()
     g.close()
+
+
+def test_refinement_that_ran_out_of_memory_can_be_repeated(ctx):
+    """A refinement whose allocations fail after its marks leaves the element set as it was, and the same
+    call with memory adds the same elements as on a grid that never failed."""
+    lib = amdg.load()
+    grids = []
+    for _ in range(2):
+        g = amdg.Grid(ctx, 3, 6, 2, level_init=3)
+        g.init_separable_adaptive(O.burgers_ic_terms(3), 1e-3)
+        grids.append(g)
+    want, g = grids
+    n = g.num_elements
+    try:
+        after, failed = 0, 0
+        while True:
+            lib.amdg_debug_fail_device_allocations(after)
+            try:
+                g.refine(1e-6)
+                break
+            except amdg.AmdgError as err:
+                assert err.status == NOMEM
+                failed += 1
+                after += 1
+        assert failed > 1
+    finally:
+        lib.amdg_debug_fail_device_allocations(-1)
+    want.refine(1e-6)
+    assert g.num_elements > n
+    assert all(np.array_equal(a, b) for a, b in zip(g.elements(), want.elements()))
+    assert np.array_equal(g.coefficients(), want.coefficients())
+    g.close()
+    want.close()
