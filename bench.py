@@ -39,8 +39,8 @@ CFL = 0.1
 # (dram__bytes_read.sum + dram__bytes_write.sum; variant 0 was not captured)
 NCU_TRAFFIC_BYTES = {1: (720.902 + 241.610) * 1e6, 2: (441.076 + 236.082) * 1e6}
 # DRAM bytes of one FP64 right-hand side of the 3D adaptive Burgers workload on its final grid
-# (1,004 elements), summed over its 11 kernels, ncu with a cold L2 before every kernel
-NCU_TRAFFIC_RHS_CONFIG3 = 24.704512e6
+# (1,004 elements), summed over its 10 kernels, ncu with a cold L2 before every kernel
+NCU_TRAFFIC_RHS_CONFIG3 = 13.66e6
 METRIC = "DOF-stage updates/s at matched L2 error: plain FP64 vs mixed+learned-adapt"
 WORKLOAD = "6D linear advection, sparse grid N=8, Alpert k=2, SSP-RK3 (34,455,456 DOF)"
 
@@ -450,7 +450,7 @@ def run_ours(args):
         "l2_error_vs_exact_l1_l2_linf": plain["error_vs_exact_l1_l2_linf"],
         "roofline": {"bound": "hbm", "achieved": ach, "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": ach / pk["hbm_gbs"], "traffic": NCU_TRAFFIC_RHS_CONFIG3, "peak_kind": pk_kind,
-                     "traffic_note": "dram__bytes_read.sum + dram__bytes_write.sum summed over the 11 kernels of one "
+                     "traffic_note": "dram__bytes_read.sum + dram__bytes_write.sum summed over the 10 kernels of one "
                                      "FP64 right-hand side on this grid, ncu with its default cache flush before "
                                      "every kernel (cold L2); in the run the working set stays in L2 "
                                      "(profiles/rhs_burgers3d_config3.md)",
@@ -1380,7 +1380,7 @@ def profile_herm():
 def profile_rhs_config3():
     """Profiling case (not a bench line): one FP64 and one mixed right-hand side on the final grid of
     a plain 3D adaptive Burgers run (1,004 elements), each after a warm-up evaluation, between
-    cudaProfilerStart / cudaProfilerStop (the dozen kernels of each, for DRAM traffic per RHS)."""
+    cudaProfilerStart / cudaProfilerStop (the ten kernels of each, for DRAM traffic per RHS)."""
     import torch
 
     import amdg
