@@ -34,7 +34,7 @@ namespace {
 
 constexpr int kSweepCta = 128;    // middle sweeps
 constexpr int kOutCta = 256;      // largest CTA of the last sweep
-constexpr int64_t kSharedEntries = 8192;  // outputs of a sweep (elements x entries) up to which four lanes share one
+constexpr int64_t kSharedEntries = 8192;  // 2D: outputs of a sweep (elements x entries) up to which four lanes share one
 constexpr int kSharedPhases = 4;
 constexpr size_t kPartBytes = 32 * 1024;  // shared memory for the products' parts
 constexpr int kLongItems = 4;     // output entries of a long row's unit in the last sweep
@@ -142,10 +142,10 @@ __device__ __forceinline__ float2 exact_dot(const float (&x)[NF], const float (&
 }
 
 // output entry idx: the neighbours beg + ph, beg + ph + P, ..., four at a time, their operands loaded
-// before the multiply-adds.  FP32 entries that several lanes share (P > 1: small grids, long rows) carry
-// the roundings of their sums along: the volume and interface parts of a right-hand side cancel, and plain
+// before the multiply-adds.  FP32 entries that several lanes share (P > 1: small grids, and long rows beside
+// columns: EXACT) carry the roundings of their sums along: the volume and interface parts of a right-hand side cancel, and plain
 // sums left the Hermite one on 256-450 elements 6 % less exact than chains of multiply-adds did.
-template <typename T, int NF, int NT>
+template <typename T, int NF, int NT, bool EXACT>
 __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, int P) {
     const int rest = quotient(idx, f.product), inner = idx - rest * f.stride;
     const T* in = f.in + (rest / NT) * NF * f.stride + inner;
@@ -182,7 +182,7 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
                     xv[j][k] = x[j][k * f.stride];
                     mv[j][k] = __ldg(mm[j] + k * NT);
                 }
-            if (P > 1) {
+            if (EXACT && P > 1) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) add(exact_dot<NF>(xv[j], mv[j]));
             } else {
@@ -236,7 +236,7 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
                 xv[k] = x[k * f.stride];
                 mv[k] = __ldg(mm + k * NT);
             }
-            if (P > 1) {
+            if (EXACT && P > 1) {
                 add(exact_dot<NF>(xv, mv));
             } else {
                 part = xv[0] * mv[0];
@@ -251,18 +251,18 @@ __device__ __forceinline__ T fibre_entry_n(const Fibre<T>& f, int idx, int ph, i
             acc = part;
         }
     }
-    if constexpr (std::is_same<T, float>::value) {
+    if constexpr (EXACT && std::is_same<T, float>::value) {
         const float whole = acc + lost;
         if (whole == whole) acc = whole;  // an overflowed sum stays infinite
     }
     return times(acc, f.product);
 }
-template <typename T, int NF, int NT>
+template <typename T, int NF, int NT, bool EXACT>
 __device__ __forceinline__ T fibre_entry(const Fibre<T>& f, int idx, int ph, int P) {
     if constexpr (NT == 3 && NF != 3) {  // the penalty product beside the transforms back
-        if (f.nf == 3) return fibre_entry_n<T, 3, NT>(f, idx, ph, P);
+        if (f.nf == 3) return fibre_entry_n<T, 3, NT, EXACT>(f, idx, ph, P);
     }
-    return fibre_entry_n<T, NF, NT>(f, idx, ph, P);
+    return fibre_entry_n<T, NF, NT, EXACT>(f, idx, ph, P);
 }
 
 // acc += one neighbour's part of a column, summed by itself first (a blocked sum: its rounding errors
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
                 T part;
                 set_zero(part);
                 if (idx < a.out_block)
-                    part = fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[p], e, shorten), idx, ph, kLongPhases);
+                    part = fibre_entry<T, NF, NT, COL || (P > 1)>(fibre_of<T, NF, NT>(a, prods[p], e, shorten), idx, ph, kLongPhases);
                 sum = add_t(sum, phase_sum<kLongPhases>(part));
             }
             if (ph == 0 && idx < a.out_block) {
@@ -449,9 +449,9 @@ __global__ void __launch_bounds__(kSweepCta, 1024 / kSweepCta) plan_sweep_kernel
         T sum;
         set_zero(sum);
         if (mine) {
-            sum = fibre_entry<T, NF, NT>(f0, item, ph, P);
+            sum = fibre_entry<T, NF, NT, COL || (P > 1)>(f0, item, ph, P);
             for (int p = 1; p < node.count; ++p)
-                sum = add_t(sum, fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[p], re, shorten), item, ph, P));
+                sum = add_t(sum, fibre_entry<T, NF, NT, COL || (P > 1)>(fibre_of<T, NF, NT>(a, prods[p], re, shorten), item, ph, P));
         }
         sum = phase_sum<P>(sum);
         if (mine && ph == 0) {
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
                     T v;
                     set_zero(v);
                     if (k < total && idx < a.out_block)
-                        v = fibre_entry<T, NF, NT>(fibre_of<T, NF, NT>(a, prods[k / kLongItems], e, shorten), idx, ph, kLongPhases);
+                        v = fibre_entry<T, NF, NT, COL || (P > 1)>(fibre_of<T, NF, NT>(a, prods[k / kLongItems], e, shorten), idx, ph, kLongPhases);
                     v = phase_sum<kLongPhases>(v);
                     if (ph == 0 && k < total) part[k] = v;
                 }
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, Pla
         } else {
             T v;
             set_zero(v);
-            if (k.live) v = fibre_entry<T, NF, NT>(f0, w0 + k.item, tid % P, P);
+            if (k.live) v = fibre_entry<T, NF, NT, COL || (P > 1)>(f0, w0 + k.item, tid % P, P);
             v = phase_sum<P>(v);
             if (k.live && tid % P == 0) y[k.item] = v;
         }
@@ -624,10 +624,13 @@ namespace {
 // lanes per output entry: on grids of few outputs a launch lasts as long as one thread's chain over its
 // rows, so four lanes share an entry.  Measured with the limit at 0 / 8 k / 24 k / 64 k outputs: adaptive
 // 2D Hermite step (190-390 elements) 514 / 436 / 433 / 434 us, adaptive 3D step (830-1,170 elements) 866 /
-// 867 / 884 / 1,116 us: beyond it the FP64 pipe is busy and the four parts' sums only add to its work.
+// 867 / 884 / 1,116 us: beyond it the FP64 pipe is busy and the four parts' sums only add to its work.  In
+// two dimensions only: with more, rows are shorter and the products, each with its own sum over the
+// lanes, more.  FP64 right-hand sides with and without sharing: 2D N = 5 29 / 44 us, N = 7 60 / 71; 3D N = 4
+// 57 / 51, 4D N = 2 139 / 67, 5D N = 1 346 / 111.
 template <typename T>
 bool shared_entries(const PlanArgs<T>& a) {
-    return a.num_elements * a.out_block <= kSharedEntries;
+    return a.dim == 2 && a.num_elements * a.out_block <= kSharedEntries;
 }
 
 template <typename T, int NF, int NT>
