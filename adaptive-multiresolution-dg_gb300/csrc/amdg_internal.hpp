@@ -281,8 +281,7 @@ struct PlanProduct {
 struct PlanNode {
     int32_t first, count;  // products
     int32_t long_dim;      // middle sweeps: the dimension of the products that are not "U" parts, -1 if none
-    int32_t long_mask;     // last sweep: the dimensions of those products, one bit each (transforms back: of all
-                           // the operator's terms, so that a group is summed alike by itself and beside others)
+    int32_t long_mask;     // last sweep: the dimensions of those products, one bit each
 };
 struct SweepPlan {
     int offset[kMaxDim] = {0}, count[kMaxDim] = {0};  // nodes of each sweep
@@ -495,9 +494,9 @@ struct amdg_burgers_op {
     amdg::PlanNode* d_plan_nodes = nullptr;
     amdg::PlanProduct* d_plan_products = nullptr;
     size_t plan_nodes_cap = 0, plan_products_cap = 0;  // bytes
-    // forms of the last sweep that change the order of its sums, chosen from all terms: FP32 columns of
-    // the transforms to points and back, and the dimensions whose long rows the transforms back share out
-    bool pv_columns = false, rhs_columns = false;
+    // forms of the last sweep of the transforms back that change the order of its sums, from all terms: FP32
+    // columns, and the dimensions whose long rows are shared out (plan_columns)
+    bool rhs_columns = false;
     int32_t rhs_long_mask = 0;
     // per sweep of the transforms to point values: the last evaluation (they are numbered) with an input
     // that was not finite.  (A step replayed as a graph keeps its numbers: after such an evaluation it

@@ -276,20 +276,15 @@ amdg_status upload_plans(amdg_burgers_op* op, cudaStream_t st) {
 SweepPlan make_plan(amdg_burgers_op* op, int first, int count) {
     const bool pv = first < op->n_pv_terms;
     const int np = op->grid->host.k + 1, dim = op->grid->host.dim;
-    const SweepPlan p = build_sweep_plan(op->terms, first, count, dim, pv ? np : op->p1, pv ? op->p1 : np, np, pv,
-                                         &op->plan_nodes, &op->plan_products);
-    for (int k = 0; !pv && k < p.count[dim - 1]; ++k)
-        op->plan_nodes[size_t(p.offset[dim - 1] + k)].long_mask = op->rhs_long_mask;
-    return p;
+    return build_sweep_plan(op->terms, first, count, dim, pv ? np : op->p1, pv ? op->p1 : np, np, pv, &op->plan_nodes,
+                            &op->plan_products);
 }
 
-// the rules of the last sweeps that the whole operator shares (amdg_burgers_op)
+// the rules of the last sweep that all terms share (amdg_burgers_op)
 void set_plan_rules(amdg_burgers_op* op) {
     const int np = op->grid->host.k + 1, dim = op->grid->host.dim, nterms = int(op->terms.size());
     std::vector<PlanNode> nodes;
     std::vector<PlanProduct> products;
-    const SweepPlan pv = build_sweep_plan(op->terms, 0, op->n_pv_terms, dim, np, op->p1, np, true, &nodes, &products);
-    op->pv_columns = plan_columns(pv.max_products, op->points);
     const SweepPlan back = build_sweep_plan(op->terms, op->n_pv_terms, nterms - op->n_pv_terms, dim, op->p1, np, np, false,
                                             &nodes, &products);
     op->rhs_columns = plan_columns(back.max_products, op->grid->block);
@@ -510,7 +505,13 @@ amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count
     a.n_out = n_out;
     a.products = op->d_plan_products;
     a.max_products = plan.max_products;
-    a.columns = first < op->n_pv_terms ? op->pv_columns : op->rhs_columns;
+    const bool pv = first < op->n_pv_terms;
+    if (!pv && int(op->terms.size()) - op->n_pv_terms <= op->chunk) {
+        a.columns = op->rhs_columns;
+        a.long_mask = op->rhs_long_mask;
+    } else {
+        a.columns = plan_columns(plan.max_products, pv ? op->points : g->block);
+    }
     for (int i = 0; i < kNumLagrMats; ++i) a.mats[i] = m.m[i];
     a.rows = static_cast<const RowRec*>(op->d_rows);
     a.vol_nbr = reinterpret_cast<const int2*>(op->d_vol_nbr);
@@ -520,7 +521,6 @@ amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count
     a.long_count = op->d_long;
     a.long_rows = op->d_long + kMaxDim;
     a.long_stride = op->long_stride;
-    const bool pv = first < op->n_pv_terms;
     const T* cur = nullptr;
     for (int j = 0; j < dim; ++j) {
         a.first_sweep = j == 0;

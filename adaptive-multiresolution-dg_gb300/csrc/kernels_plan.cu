@@ -335,7 +335,7 @@ __device__ __forceinline__ void fibre_column(const Fibre<T>& f, int c, T (&acc)[
 }
 
 // whether element e's row along the node's non-"U" dimension (middle sweeps) or one of them (last
-// sweep; of the transforms back, one of the operator's) is long
+// sweep) is long
 template <typename T>
 __device__ __forceinline__ bool long_row(const PlanArgs<T>& a, const PlanNode& node, int64_t e) {
     for (int t = 0; t < a.dim; ++t)
@@ -516,7 +516,8 @@ __device__ __forceinline__ void plan_epilogue(const PlanArgs<T>& a, const PlanOu
 template <typename T, int NF, int NT, bool COL, int P>
 __global__ void __launch_bounds__(kOutCta, 4) plan_out_kernel(PlanArgs<T> a, PlanOut o, int G, int W) {
     const int field = blockIdx.y;
-    const PlanNode node = a.nodes[field];
+    PlanNode node = a.nodes[field];
+    if (a.long_mask) node.long_mask = a.long_mask;
     const PlanProduct* prods = a.products + node.first;
     const int np = node.count;
     extern __shared__ __align__(16) unsigned char smem[];

@@ -53,6 +53,7 @@ struct PlanArgs {
     const PlanProduct* products;
     int num_nodes, max_products;     // products of the largest node
     bool columns;                    // last sweep, FP32: a thread per column (plan_columns)
+    int32_t long_mask;               // last sweep: dimensions whose long rows are shared out (0: the node's)
     int out_block;                   // output entries per element
     bool first_sweep;                // products read src[in], else in + in * in_slice
     const T* mats[kNumLagrMats];     // blocked by order pair
@@ -84,8 +85,10 @@ cudaError_t launch_plan_sweep(const PlanArgs<T>& a, cudaStream_t st);
 template <typename T>
 cudaError_t launch_plan_out(const PlanArgs<T>& a, const PlanOut& o, cudaStream_t st);
 // whether the FP32 last sweep of nodes of up to max_products products takes a thread per column: where an
-// element's parts fit the shared memory.  The two forms add the neighbours in different orders, so an
-// operator decides once, from all its terms, and its term groups by themselves follow that.
+// element's parts fit the shared memory.  The two forms add the neighbours in different orders: where all
+// terms of an operator go in one launch sequence, it decides from all of them (as which rows are shared
+// out), and its term groups by themselves follow that; where they go in pieces, a group runs in the same
+// pieces by itself and beside the others, and the piece decides (6D Burgers, 138 elements, mixed: 3185 -> 2976 us).
 bool plan_columns(int max_products, int out_block);
 
 // row records of host-built neighbour lists (vol_skip: finer vol neighbours without a point), long rows
