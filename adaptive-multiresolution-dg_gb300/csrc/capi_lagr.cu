@@ -478,11 +478,12 @@ amdg_status run_terms(amdg_burgers_op* op, const Mats<T>& m, int first, int coun
 // the mark of the inputs of sweep j of the transforms to point values, in the current evaluation
 NonfiniteMark input_mark(const amdg_burgers_op* op, int j) { return NonfiniteMark{op->d_nonfinite + j, op->evaluation}; }
 
-// begins an evaluation of point values of the FP64 state u
-amdg_status begin_evaluation(amdg_burgers_op* op, const double* u, cudaStream_t st) {
+// begins an evaluation of point values of the state u
+template <typename T>
+amdg_status begin_evaluation(amdg_burgers_op* op, const T* u, cudaStream_t st) {
     ++op->evaluation;
     if (!planned(op)) return AMDG_OK;
-    AMDG_CK(launch_find_nonfinite(u, op->grid->dof, input_mark(op, 0), st));
+    AMDG_CK(launch_find_nonfinite<T>(u, op->grid->dof, input_mark(op, 0), st));
     op->grid->ctx->launches++;
     return AMDG_OK;
 }
@@ -524,8 +525,7 @@ amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count
     const T* cur = nullptr;
     for (int j = 0; j < dim; ++j) {
         a.first_sweep = j == 0;
-        // (nothing has looked through the FP32 state of amdg_burgers_point_values and _flux_coefficients)
-        a.in_mark = pv && (j > 0 || !std::is_same<T, float>::value) ? input_mark(op, j) : NonfiniteMark{};
+        a.in_mark = pv ? input_mark(op, j) : NonfiniteMark{};
         a.out_mark = pv && j + 1 < dim ? input_mark(op, j + 1) : NonfiniteMark{};
         a.in = cur;
         a.in_slice = j == 0 ? 0 : E * ipow(n_out, j) * ipow(n_in, dim - j);
@@ -554,11 +554,7 @@ amdg_status eval_point_values(amdg_burgers_op* op, const Mats<T>& m, const T* u,
     const bool herm = op->kind == 3;  // the Hermite flux needs the slopes too: applied after the sum
     T* slots = static_cast<T*>(op->w_slots);
     const T* src[1] = {u};
-    if constexpr (std::is_same<T, double>::value) {
-        if (amdg_status r = begin_evaluation(op, u, st); r != AMDG_OK) return r;
-    } else {
-        ++op->evaluation;
-    }
+    if (amdg_status r = begin_evaluation(op, u, st); r != AMDG_OK) return r;
     if (planned(op)) {
         const auto ranges = term_ranges(op, 0, op->n_pv_terms);
         for (size_t i = 0; i < ranges.size(); ++i) {

@@ -633,16 +633,20 @@ template cudaError_t launch_reduce_points_coef<double>(const double*, int, int64
 template cudaError_t launch_reduce_points_coef<float2>(const float2*, int, int64_t, int, int, const int32_t*,
                                                        const double*, double, double*, cudaStream_t);
 
-__global__ void find_nonfinite_kernel(const double* u, int64_t n, NonfiniteMark mark) {
+template <typename T>
+__global__ void find_nonfinite_kernel(const T* u, int64_t n, NonfiniteMark mark) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     wait_for_previous();
     if (i < n) note(mark, u[i]);
 }
 
-cudaError_t launch_find_nonfinite(const double* u, int64_t n, NonfiniteMark mark, cudaStream_t st) {
+template <typename T>
+cudaError_t launch_find_nonfinite(const T* u, int64_t n, NonfiniteMark mark, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    return launch_after(find_nonfinite_kernel, AMDG_EW_AFTER(n), u, n, mark);
+    return launch_after(find_nonfinite_kernel<T>, AMDG_EW_AFTER(n), u, n, mark);
 }
+template cudaError_t launch_find_nonfinite<double>(const double*, int64_t, NonfiniteMark, cudaStream_t);
+template cudaError_t launch_find_nonfinite<float>(const float*, int64_t, NonfiniteMark, cudaStream_t);
 
 // the high parts by themselves (hi, unless null) are the FP32 state that the penalty reads
 __global__ void to_df_kernel(const double* in, float2* out, float* hi, int64_t n, NonfiniteMark mark) {

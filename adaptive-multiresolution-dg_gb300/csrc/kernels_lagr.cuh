@@ -73,7 +73,8 @@ __device__ __forceinline__ void note(const NonfiniteMark& m, T v) {
 }
 #endif
 // note(mark, u[i]) for n entries
-cudaError_t launch_find_nonfinite(const double* u, int64_t n, NonfiniteMark mark, cudaStream_t st);
+template <typename T>
+cudaError_t launch_find_nonfinite(const T* u, int64_t n, NonfiniteMark mark, cudaStream_t st);
 
 // double -> double-float (hi = float(v), lo = float(v - hi))
 cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, NonfiniteMark mark, cudaStream_t st);
