@@ -503,6 +503,8 @@ struct amdg_burgers_op {
     // takes the whole lists until it is captured again.)
     uint32_t* d_nonfinite = nullptr;
     uint32_t evaluation = 0;
+    uint32_t noted = 0;        // number under which the first sweep's mark tells about the current evaluation's state
+    uint32_t state_noted = 0;  // ... and about the grid's coefficients, inside a step that has looked (0: not known)
     void* d_rows = nullptr;          // amdg::RowRec per (element, dimension)
     int32_t* d_long = nullptr;       // long rows: counts per dimension (kMaxDim), then the elements per dimension
     int64_t long_stride = 0;

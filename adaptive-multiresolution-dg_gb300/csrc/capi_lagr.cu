@@ -476,13 +476,20 @@ amdg_status run_terms(amdg_burgers_op* op, const Mats<T>& m, int first, int coun
 }
 
 // the mark of the inputs of sweep j of the transforms to point values, in the current evaluation
-NonfiniteMark input_mark(const amdg_burgers_op* op, int j) { return NonfiniteMark{op->d_nonfinite + j, op->evaluation}; }
+NonfiniteMark input_mark(const amdg_burgers_op* op, int j) {
+    return NonfiniteMark{op->d_nonfinite + j, j == 0 ? op->noted : op->evaluation};
+}
 
-// begins an evaluation of point values of the state u
+// the mark for a state that the next evaluation reads
+NonfiniteMark next_mark(const amdg_burgers_op* op) { return NonfiniteMark{op->d_nonfinite, op->evaluation + 1}; }
+
+// Begins an evaluation of point values of the state u.  noted: the number under which the mark of the first
+// sweep already tells whether u is finite (0: u is looked through)
 template <typename T>
-amdg_status begin_evaluation(amdg_burgers_op* op, const T* u, cudaStream_t st) {
+amdg_status begin_evaluation(amdg_burgers_op* op, const T* u, uint32_t noted, cudaStream_t st) {
     ++op->evaluation;
-    if (!planned(op)) return AMDG_OK;
+    op->noted = noted ? noted : op->evaluation;
+    if (noted || !planned(op)) return AMDG_OK;
     AMDG_CK(launch_find_nonfinite<T>(u, op->grid->dof, input_mark(op, 0), st));
     op->grid->ctx->launches++;
     return AMDG_OK;
@@ -548,13 +555,14 @@ amdg_status run_plan(amdg_burgers_op* op, const Mats<T>& m, int first, int count
 // u_h at the interpolation points (FP64 or FP32 arithmetic): into up, or, when
 // fp is given, f(u) = u^2/2 at the points into fp
 template <typename T>
-amdg_status eval_point_values(amdg_burgers_op* op, const Mats<T>& m, const T* u, T* up, T* fp, cudaStream_t st) {
+amdg_status eval_point_values(amdg_burgers_op* op, const Mats<T>& m, const T* u, T* up, T* fp, cudaStream_t st,
+                              uint32_t noted = 0) {
     const int np = op->grid->host.k + 1;
     const int64_t n = op->grid->host.num_elements * op->points;
     const bool herm = op->kind == 3;  // the Hermite flux needs the slopes too: applied after the sum
     T* slots = static_cast<T*>(op->w_slots);
     const T* src[1] = {u};
-    if (amdg_status r = begin_evaluation(op, u, st); r != AMDG_OK) return r;
+    if (amdg_status r = begin_evaluation(op, u, noted, st); r != AMDG_OK) return r;
     if (planned(op)) {
         const auto ranges = term_ranges(op, 0, op->n_pv_terms);
         for (size_t i = 0; i < ranges.size(); ++i) {
@@ -590,7 +598,7 @@ amdg_status eval_point_values_df(amdg_burgers_op* op, const double* u, double* u
     const int np = op->grid->host.k + 1;
     const int64_t n = op->grid->host.num_elements * op->points;
     float2* udf = static_cast<float2*>(op->w_u);
-    ++op->evaluation;
+    op->noted = ++op->evaluation;
     AMDG_CK(launch_to_df(u, udf, u32, op->grid->dof, input_mark(op, 0), st));
     op->grid->ctx->launches++;
     float2* slots = static_cast<float2*>(op->w_slots);
@@ -723,7 +731,7 @@ amdg_status eval_wave_penalty(amdg_burgers_op* op, const double* u, double* rhs,
 // coefficients (type To) into fields dim+1 .. 2 dim+1 of w_fields
 template <typename To>
 amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, cudaStream_t st, int f_first = 0,
-                             int f_last = -1, float* u32 = nullptr) {
+                             int f_last = -1, float* u32 = nullptr, uint32_t noted = 0) {
     amdg_grid* g = op->grid;
     const int dim = g->host.dim, np = g->host.k + 1;
     const int64_t E = g->host.num_elements, n = E * op->points;
@@ -736,12 +744,12 @@ amdg_status eval_wave_fields(amdg_burgers_op* op, const double* u, To** fucoe, c
     Tp* slots = static_cast<Tp*>(op->w_slots);
     const Tp* src[1];
     if constexpr (df) {
-        ++op->evaluation;
+        op->noted = ++op->evaluation;
         AMDG_CK(launch_to_df(u, static_cast<float2*>(op->w_u), u32, g->dof, input_mark(op, 0), st));
         op->grid->ctx->launches++;
         src[0] = static_cast<const float2*>(op->w_u);
     } else {
-        if (amdg_status r = begin_evaluation(op, u, st); r != AMDG_OK) return r;
+        if (amdg_status r = begin_evaluation(op, u, noted, st); r != AMDG_OK) return r;
         src[0] = u;
     }
     const Mats<Tp> m = [&] {
@@ -837,7 +845,9 @@ float* state32(amdg_burgers_op* op) {
 // fine-level surpluses are small differences of O(1) point values, which FP32
 // rounding would swamp.  In mixed mode the back transforms (the bulk of the
 // work) and the penalty run in FP32, their terms summed in FP64.
-amdg_status eval_rhs(amdg_burgers_op* op, const double* u, double* rhs, amdg_precision prec, StageOut so = StageOut{}) {
+// noted: as begin_evaluation (FP64).
+amdg_status eval_rhs(amdg_burgers_op* op, const double* u, double* rhs, amdg_precision prec, StageOut so = StageOut{},
+                     uint32_t noted = 0) {
     PhaseTimer timer(op->grid->ctx, AMDG_PHASE_RHS);
     cudaStream_t st = stream_of(op);
     const int dim = op->grid->host.dim;
@@ -847,7 +857,7 @@ amdg_status eval_rhs(amdg_burgers_op* op, const double* u, double* rhs, amdg_pre
         if (prec == AMDG_PREC_FP64) {
             double* fc[kMaxTermSources];
             for (int f = 0; f <= dim; ++f) fc[f] = fields + size_t(dim + 1 + f) * stride;
-            if (amdg_status r = eval_wave_fields<double>(op, u, fc, st); r != AMDG_OK) return r;
+            if (amdg_status r = eval_wave_fields<double>(op, u, fc, st, 0, -1, nullptr, noted); r != AMDG_OK) return r;
             return eval_back_transforms<double>(op, mats64(op), fc, dim + 1, u, rhs, so, st);
         }
         float* fc[kMaxTermSources];
@@ -858,7 +868,7 @@ amdg_status eval_rhs(amdg_burgers_op* op, const double* u, double* rhs, amdg_pre
     }
     double* fp = static_cast<double*>(op->w_a);
     amdg_status r = prec == AMDG_PREC_FP64
-                        ? eval_point_values<double>(op, mats64(op), u, static_cast<double*>(op->w_up), fp, st)
+                        ? eval_point_values<double>(op, mats64(op), u, static_cast<double*>(op->w_up), fp, st, noted)
                         : eval_point_values_df(op, u, static_cast<double*>(op->w_up), fp, st, state32(op));
     if (r != AMDG_OK) return r;
     if (prec == AMDG_PREC_FP64) {
@@ -1454,12 +1464,16 @@ amdg_status amdg_burgers_rk3_steps(amdg_burgers_op* op, double dt, int nsteps, a
     if (nsteps == 0) return AMDG_OK;
     // one step: u^n stays in the grid's coefficients until the last stage writes them; a stage's output
     // is another vector than its input, which the last sweep reads at neighbouring elements
-    auto step = [&]() -> amdg_status {
+    // FP64: a stage notes what is not finite of the state that the next one reads
+    auto step = [&](uint32_t noted) -> amdg_status {
         double* const in[3] = {g->d_u, op->d_u1, op->d_u2};
         double* const out[3] = {op->d_u1, op->d_u2, g->d_u};
         for (int stage = 0; stage < 3; ++stage) {
-            const StageOut so{1, stage_coef(stage, dt), g->d_u, in[stage], out[stage]};
-            if (amdg_status r = eval_rhs(op, in[stage], op->d_rhs64, prec, so); r != AMDG_OK) return r;
+            StageOut so{1, stage_coef(stage, dt), g->d_u, in[stage], out[stage], NonfiniteMark{}};
+            const bool note_out = prec == AMDG_PREC_FP64 && planned(op) && stage < 2;
+            if (note_out) so.mark = NonfiniteMark{op->d_nonfinite, op->evaluation + 2};  // of the next evaluation but this
+            if (amdg_status r = eval_rhs(op, in[stage], op->d_rhs64, prec, so, noted); r != AMDG_OK) return r;
+            noted = note_out ? op->evaluation + 1 : 0;
         }
         return AMDG_OK;
     };
@@ -1475,14 +1489,14 @@ amdg_status amdg_burgers_rk3_steps(amdg_burgers_op* op, double dt, int nsteps, a
     op->last_version = g->version;
     op->last_prec = int(prec);
     op->last_dt = dt;
-    if (!graph_valid && nsteps == 1 && !repeat) return step();
+    if (!graph_valid && nsteps == 1 && !repeat) return step(op->state_noted);
     if (!graph_valid) {
         if (op->graph_exec) cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(op->graph_exec));
         op->graph_exec = nullptr;
         const int64_t l0 = g->ctx->launches;
         cudaGraph_t graph = nullptr;
         AMDG_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        const amdg_status r = step();
+        const amdg_status r = step(0);  // a replayed step looks through its state
         cudaError_t ec = cudaStreamEndCapture(st, &graph);
         op->graph_launches = g->ctx->launches - l0;
         g->ctx->launches = l0;
@@ -1553,7 +1567,7 @@ static amdg_status adaptive_step_any(amdg_burgers_op* op, double cfl, double wav
     if (burgers_like(op)) {
         op->rhs_evaluations++;
         // forward Euler into the prediction buffer (ForwardEuler::step_stage)
-        const StageOut so{1, stage_coef(0, dt), g->d_u, g->d_u, op->d_pred};
+        const StageOut so{1, stage_coef(0, dt), g->d_u, g->d_u, op->d_pred, NonfiniteMark{}};
         if ((s = eval_rhs(op, g->d_u, op->d_rhs64, prec, so)) != AMDG_OK) return s;
     } else {
         // EulerODE2nd::step_rk_source on copies of (u, v): u + dt v, v + dt (IPDG u)
@@ -1575,7 +1589,11 @@ static amdg_status adaptive_step_any(amdg_burgers_op* op, double cfl, double wav
                 return s;
             if (decisions) std::copy(refined.begin(), refined.end(), decisions);
         }
-        if ((s = one_step(op, dt, prec)) != AMDG_OK) return s;
+        // the step begins from the coefficients that the predictor looked through; refining copied them and added zeros
+        op->state_noted = burgers_like(op) && prec == AMDG_PREC_FP64 && planned(op) ? op->noted : 0;
+        s = one_step(op, dt, prec);
+        op->state_noted = 0;
+        if (s != AMDG_OK) return s;
         if ((s = grid_coarsen(g, eta, op->kind == 1 ? g->d_v : nullptr, nullptr)) != AMDG_OK) return s;
         if (decisions) {
             if ((s = grid_ensure_host(g)) != AMDG_OK) return s;
@@ -1975,10 +1993,14 @@ static amdg_status wave_rk4(amdg_burgers_op* op, double dt, int nsteps, amdg_pre
     for (int step = 0; step < nsteps; ++step) {
         AMDG_CK(cudaMemcpyAsync(op->d_u1, g->d_u, bytes, cudaMemcpyDeviceToDevice, st));
         AMDG_CK(cudaMemcpyAsync(op->d_v1, g->d_v, bytes, cudaMemcpyDeviceToDevice, st));
+        uint32_t noted = 0;
         for (int stage = 0; stage < 4; ++stage) {
-            if (amdg_status r = eval_rhs(op, op->d_u1, op->d_rhs64, prec); r != AMDG_OK) return r;
+            if (amdg_status r = eval_rhs(op, op->d_u1, op->d_rhs64, prec, StageOut{}, noted); r != AMDG_OK) return r;
+            const bool note_out = prec == AMDG_PREC_FP64 && planned(op) && stage < 3;
+            const NonfiniteMark mark = note_out ? next_mark(op) : NonfiniteMark{};
+            noted = note_out ? mark.evaluation : 0;
             AMDG_CK(launch_rk4_2nd_stage(stage, dt, op->d_rhs64, g->d_u, g->d_v, op->d_u1, op->d_v1, op->d_su, op->d_sv,
-                                         g->dof, st));
+                                         g->dof, st, mark));
             g->ctx->launches++;
         }
         op->rhs_evaluations += 4;

@@ -666,7 +666,7 @@ cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, No
 
 // Eigen evaluates each vector expression elementwise with one rounding per operation (no contraction)
 __global__ void rk4_2nd_stage_kernel(int stage, double dt, const double* rhs, double* un, double* vn, double* us,
-                                     double* vs, double* su, double* sv, int64_t n) {
+                                     double* vs, double* su, double* sv, int64_t n, NonfiniteMark mark) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     wait_for_previous();
     if (i >= n) return;
@@ -694,13 +694,16 @@ __global__ void rk4_2nd_stage_kernel(int stage, double dt, const double* rhs, do
         const double tu = __dadd_rn(su[i], ku), tv = __dadd_rn(sv[i], kv);
         un[i] = __dadd_rn(un[i], __dmul_rn(1. / 6., tu));
         vn[i] = __dadd_rn(vn[i], __dmul_rn(1. / 6., tv));
+        return;
     }
+    note(mark, us[i]);
 }
 
 cudaError_t launch_rk4_2nd_stage(int stage, double dt, const double* rhs, double* un, double* vn, double* us, double* vs,
-                                 double* su, double* sv, int64_t n, cudaStream_t st) {
+                                 double* su, double* sv, int64_t n, cudaStream_t st,
+                                 NonfiniteMark mark) {
     if (n == 0) return cudaSuccess;
-    return launch_after(rk4_2nd_stage_kernel, AMDG_EW_AFTER(n), stage, dt, rhs, un, vn, us, vs, su, sv, n);
+    return launch_after(rk4_2nd_stage_kernel, AMDG_EW_AFTER(n), stage, dt, rhs, un, vn, us, vs, su, sv, n, mark);
 }
 
 }  // namespace amdg

@@ -84,7 +84,7 @@ cudaError_t launch_to_df(const double* in, float2* out, float* hi, int64_t n, No
 // (su, sv); stage 3 writes un + su/6, vn + sv/6 into (un, vn).  EulerODE2nd (stage -1):
 // out_u = un + dt vn, out_v = vn + dt rhs into (us, vs).
 cudaError_t launch_rk4_2nd_stage(int stage, double dt, const double* rhs, double* un, double* vn, double* us, double* vs,
-                                 double* su, double* sv, int64_t n, cudaStream_t st);
+                                 double* su, double* sv, int64_t n, cudaStream_t st, NonfiniteMark mark = {});
 
 // Right-hand side: v = (first ? 0 : acc) + sum_s buf[s] (in order, in FP64);
 // not last: acc = v; last: out = rk_combine(rk, un, us, v) when stage is set,
@@ -95,6 +95,7 @@ struct StageOut {
     const double* un;
     const double* us;
     double* out;
+    NonfiniteMark mark;  // of the updated state (planned FP64 sweeps)
 };
 template <typename T>
 cudaError_t launch_reduce_rhs(const T* buf, int count, int64_t n, int first, int last, double* acc, StageOut so,

@@ -47,7 +47,8 @@ __device__ __forceinline__ void set_zero(float2& v) { v = make_float2(0.0f, 0.0f
 // Whether a transform to point values may stop before a row's zero blocks: all inputs of the sweep are
 // finite.  A block of zeros times a value that is not finite is NaN, and over the whole list it reaches
 // the points that it reaches in the sweeps term by term.  Every writer of such inputs notes them; the
-// look at the state costs an FP64 right-hand side 1 to 2 %, whole lists in all sweeps 5 to 8 %.
+// look at the state costs a single FP64 right-hand side 1 to 2 %, of a step (one look, the stages note their
+// outputs) 0.5 to 1 %; whole lists in all sweeps would cost 5 to 8 %.
 template <typename T>
 __device__ __forceinline__ bool inputs_finite(const PlanArgs<T>& a) {
     return a.in_mark.at && *static_cast<const volatile uint32_t*>(a.in_mark.at) != a.in_mark.evaluation;
@@ -502,7 +503,9 @@ __device__ __forceinline__ void plan_epilogue(const PlanArgs<T>& a, const PlanOu
         const double c = 1.0 + o.amp * prod;
         static_cast<double*>(o.out[field])[i] = (c * c) * v;
     } else if (o.mode == kEpiRhs && o.last && o.so.fused) {
-        o.so.out[i] = rk_combine(o.so.rk.a, o.so.un[i], o.so.rk.b, o.so.us[i], o.so.rk.dt, v);
+        const double next = rk_combine(o.so.rk.a, o.so.un[i], o.so.rk.b, o.so.us[i], o.so.rk.dt, v);
+        o.so.out[i] = next;
+        if constexpr (std::is_same<T, double>::value) note(o.so.mark, next);
     } else {
         acc[i] = v;
     }

@@ -79,3 +79,28 @@ def test_steps_spread_them_alike(ctx, kind, dim, nmax, prec):
     assert np.isfinite(outs[-1, "first"]).all()
     assert np.array_equal(outs[-1, "first"], outs[-1, "again"])
     g.close()
+
+
+@pytest.mark.parametrize("hermite", [False, True])
+def test_stages_that_overflow_spread_alike(ctx, hermite):
+    """One FP64 step from a finite state with one coefficient so large that its square is near the largest
+    double: the stages overflow, and the later ones read what the earlier ones wrote (the look at the state
+    found nothing).  The same entries are not finite as with the sweeps term by term."""
+    g = amdg.Grid(ctx, 2, 6, 2)
+    u = np.random.default_rng(9).standard_normal((g.num_elements, g.block))
+    levels, _ = g.elements()
+    fine = np.flatnonzero(np.asarray(levels).reshape(g.num_elements, 2)[:, 0] == 5)[2]
+    outs = []
+    for variant in (-1, 0):
+        v = u.copy()
+        v[fine, 1] = 1e153
+        g.set_coefficients(v)
+        op = amdg.BurgersOperator(g, 0.825, hermite=hermite)
+        op.set_sweep_variant(variant)
+        op.rk3_steps(1e-3, 1)
+        ctx.synchronize()
+        outs.append(g.coefficients().copy())
+        op.close()
+    assert not np.isfinite(outs[1]).all()
+    assert np.array_equal(np.isfinite(outs[0]), np.isfinite(outs[1]))
+    g.close()
